@@ -108,8 +108,8 @@ typedef struct {
     int order;       /* pac_order, default PAC_ORDER_REFERENCE */
     /* 1: pick launch shapes by measurement.  The context's first passes
        each try one candidate shape (blocks per SM of the tetrahedron
-       enumeration and scan kernels, rows of a large ball per enumeration
-       work unit, queue entries a scan warp claims; 12 candidates), timing
+       enumeration and scan kernels, queue entries a scan warp claims; 12
+       candidates), timing
        the tetrahedron stage; later passes use the fastest.  Every shape
        gives the same lists, so tuning passes return correct results too. */
     int autotune;
@@ -117,15 +117,16 @@ typedef struct {
                         the tetrahedron stage, its counts and times to stderr */
     /* Launch-shape overrides, each used when > 0 (any of them turns the
        autotuner off): reserved_i[0] blocks per SM of the enumeration of
-       balls with at most 64 upper neighbours (default 4), [1] of the
-       orthosphere scan (4), [2] of the enumeration of larger balls (4),
-       [3] rows of a large ball per work unit (8), [4] queue entries a scan
-       warp claims (256).
+       balls with at most 64 upper neighbours (default 6), [1] of the
+       orthosphere scan (4), [2] of the enumeration of larger balls (2), [3]
+       no effect (accepted; an earlier enumeration's work units), [4] queue
+       entries a scan warp claims (256).
        reserved_i[5] = 1: no early refutation in the enumeration (every
        alpha tetrahedron goes to the scan; same lists).
-       reserved_i[6] = 1: verify mode -- the scan also replays the
-       reference's arithmetic for every decision the certified filter takes
-       and counts disagreements (pac_stats.cert_disagreements; 0 expected).
+       reserved_i[6] = 1: verify mode -- the enumeration and the scan also
+       replay the reference's arithmetic (exact mode: the exact polynomials)
+       for every decision that their certified filters take and count
+       disagreements (pac_stats.cert_disagreements; 0 expected).
        reserved_i[7] = W > 1, reserved_i[8] = r: slab r of W of one molecule
        (as written only): the pass outputs the simplices whose smallest
        vertex in cell order lies in the r-th of W contiguous ranges of the
@@ -137,7 +138,7 @@ typedef struct {
     int reserved_i[9];
     /* reserved_u[0]: if nonzero, the number of alpha tetrahedra the pass
        queues per chunk (default: a quarter of free device memory, at most
-       12 GiB, 32 B per entry).  Smaller values force more chunks. */
+       12 GiB, 8 B per entry).  Smaller values force more chunks. */
     uint64_t reserved_u[8];
 } pac_options;
 

@@ -63,7 +63,7 @@ def build(verbose=False, ptxas_info=False):
                                      os.path.join(SRC, "pipeline.cu")],
          [os.path.join(SRC, "pipeline.cu")] + hdrs),
         (os.path.join(OBJ, "pipeline_fma.o"),
-         [NVCC] + NVFLAGS + extra + ["-fmad=true", "-DPAC_NS=pac_fma", "-c",
+         [NVCC] + NVFLAGS + extra + ["-fmad=true", "-DPAC_NS=pac_fma", "-DPAC_CONTRACTED=1", "-c",
                                      os.path.join(SRC, "pipeline.cu")],
          [os.path.join(SRC, "pipeline.cu")] + hdrs),
         (os.path.join(OBJ, "union_measure.o"),

@@ -47,7 +47,9 @@
 // Every quantity on the left is bounded from below and on the right from
 // above, each computed in binary32 with a margin S = 1 + 2^-10 that covers
 // the rounding of the bound computations themselves; sizes outside
-// delta < 1000, W < 10^6 are never certified.
+// delta < 1000, W < 10^6 are never certified.  The weights' own rounding
+// (fl(r^2) against r^2) is inside the bounds of s_k and pi, so a certified
+// decision is also the exact one (sign of the polynomial at weights r^2).
 #pragma once
 
 #include <cmath>
@@ -110,7 +112,7 @@ PAC_CERT_FN Insphere setup(float ax, float ay, float az, float wa, float bx, flo
         const float ex = px[k] - cx, ey = py[k] - cy, ez = pz[k] - cz;
         const float d2 = ex * ex + ey * ey + ez * ez;
         s[k] = d2 - pw[k];
-        e[k] = 7.0f * kU * (d2 + pw[k]) * kS + 1e-30f;
+        e[k] = 8.0f * kU * (d2 + pw[k]) * kS + 1e-30f;
         m = fmaxf(m, fmax3(fabsf(ex), fabsf(ey), fabsf(ez)));
     }
     float rmax = e[0];
@@ -140,7 +142,7 @@ PAC_CERT_FN int test(const Insphere &c, float ex, float ey, float ez, float we) 
     if (!(del < kMaxDelta)) return -1;
     const float del2 = del * del;
     const float rhs = del * del2 * (c.k0 + c.k2 * del2) + c.kabs;
-    const float epi = 8.0f * kU * kS * (d2 + we + c.arho) + 1e-30f;
+    const float epi = 9.0f * kU * kS * (d2 + we + c.arho) + 1e-30f;
     if (fabsf(pi) - epi > rhs) return pi < 0.0f ? 1 : 0;
     return -1;
 }

@@ -65,6 +65,20 @@ int list_to_host_async(Ctx &c, int which, const uint32_t *src, size_t count, uin
     return PAC_OK;
 }
 
+int side_stream(Ctx &c) {
+    if (c.side) return PAC_OK;
+    for (auto &ev : c.side_ev)
+        if (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
+            ev = nullptr;
+            return set_error(PAC_ERR_CUDA, "cudaEventCreate (side stream) failed");
+        }
+    if (cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking) != cudaSuccess) {
+        c.side = nullptr;
+        return set_error(PAC_ERR_CUDA, "cudaStreamCreate (side stream) failed");
+    }
+    return PAC_OK;
+}
+
 int copies_join(Ctx &c) {
     if (!c.copy_stream) return PAC_OK;
     cudaError_t e = cudaEventRecord(c.copy_ev[3], c.copy_stream);
@@ -168,14 +182,12 @@ __global__ void k_check_finite(const float4 *b, uint64_t n, int *bad) {
 }
 
 // Launch shapes for the autotuner (pac_options.autotune): blocks per SM of
-// the two tetrahedron enumeration kernels and of the orthosphere scan, the
-// rows of a large ball per enumeration work unit, and the queue entries a
-// scan warp claims at a time.  The first is the default.  None of them
-// changes the output.
+// the tetrahedron enumeration (balls of at most 64 upper neighbours; larger
+// ones) and of the orthosphere scan, and the queue entries a scan warp claims
+// at a time.  The first is the default.  None of them changes the output.
 constexpr pac::LaunchShape kShapes[] = {
-    {4, 4, 4, 8, 256},  {3, 4, 4, 8, 256}, {2, 4, 4, 8, 256},  {4, 3, 4, 8, 256},
-    {4, 4, 3, 8, 256},  {4, 4, 6, 8, 256}, {4, 4, 4, 4, 256},  {4, 4, 4, 16, 256},
-    {4, 4, 4, 8, 512},  {4, 4, 4, 8, 2048}, {2, 2, 2, 8, 256}, {4, 2, 4, 4, 256}};
+    {6, 2, 4, 256}, {5, 2, 4, 256}, {4, 2, 4, 256}, {6, 1, 4, 256}, {6, 2, 3, 256}, {6, 2, 6, 256},
+    {6, 2, 4, 128}, {6, 2, 4, 512}, {6, 2, 4, 2048}, {12, 4, 4, 256}, {4, 1, 2, 256}, {6, 4, 4, 64}};
 constexpr int kNumShapes = (int)(sizeof(kShapes) / sizeof(kShapes[0]));
 static_assert(kNumShapes <= 16, "Tuner holds 16 timings");
 
@@ -198,15 +210,15 @@ int run(pac_ctx *ctx, const float4 *d_balls, uint64_t n, uint32_t n_mol,
         return pac::set_error(PAC_ERR_CUDA, std::string("input check: ") + cudaGetErrorString(e));
     if (hbad) return pac::set_error(PAC_ERR_INVALID_ARG, "non-finite ball coordinate or radius");
     // the alpha-tetrahedron queue: a quarter of the free memory at the
-    // context's first pass, at most 12 GiB (32 B per entry); a pass whose
+    // context's first pass, at most 12 GiB (8 B per entry); a pass whose
     // queued tetrahedra exceed it runs in chunks
     if (!c.queue_bytes) {
         size_t freeb = 0, totalb = 0;
         cudaMemGetInfo(&freeb, &totalb);
-        c.queue_bytes = std::max<uint64_t>(std::min<uint64_t>(freeb / 4, 12ull << 30), 32ull << 16);
+        c.queue_bytes = std::max<uint64_t>(std::min<uint64_t>(freeb / 4, 12ull << 30), 8ull << 16);
     }
     uint64_t qbytes = c.queue_bytes;
-    if (c.opt.reserved_u[0]) qbytes = c.opt.reserved_u[0] * 32ull;  // test hook: entries
+    if (c.opt.reserved_u[0]) qbytes = c.opt.reserved_u[0] * 8ull;  // test hook: entries
     const pac::LaunchShape *shape = &kShapes[0];
     // launch shapes: the caller's overrides, else the autotuner's current
     // candidate or its choice, else the defaults
@@ -221,7 +233,7 @@ int run(pac_ctx *ctx, const float4 *d_balls, uint64_t n, uint32_t n_mol,
     cfg.formula = c.opt.formula;
     cfg.tet_mode = c.opt.tet_mode;
     cfg.verbose = c.opt.verbose;
-    cfg.queue_entries = qbytes / 32;
+    cfg.queue_entries = qbytes / 8;
     cfg.exact = c.opt.predicates == PAC_PRED_EXACT;
     cfg.refute = c.opt.reserved_i[5] != 1;
     cfg.slab_world = c.opt.reserved_i[7] > 1 ? c.opt.reserved_i[7] : 1;
@@ -230,7 +242,6 @@ int run(pac_ctx *ctx, const float4 *d_balls, uint64_t n, uint32_t n_mol,
     cfg.enum_blocks = c.opt.reserved_i[0] > 0 ? c.opt.reserved_i[0] : shape->enum_blocks;
     cfg.scan_blocks = c.opt.reserved_i[1] > 0 ? c.opt.reserved_i[1] : shape->scan_blocks;
     cfg.heavy_blocks = c.opt.reserved_i[2] > 0 ? c.opt.reserved_i[2] : shape->heavy_blocks;
-    cfg.unit_rows = c.opt.reserved_i[3] > 0 ? c.opt.reserved_i[3] : shape->unit_rows;
     cfg.scan_claim = c.opt.reserved_i[4] > 0 ? c.opt.reserved_i[4] : shape->scan_claim;
     pac_stats local;
     pac_stats *sp = st ? st : &local;
@@ -242,6 +253,7 @@ int run(pac_ctx *ctx, const float4 *d_balls, uint64_t n, uint32_t n_mol,
     // a pass that stopped early may have list copies in flight: they end
     // before the pool or the pinned regions are reused
     if (rc != PAC_OK && c.copy_stream) cudaStreamSynchronize(c.copy_stream);
+    if (rc != PAC_OK && c.side) cudaStreamSynchronize(c.side);
     if (rc == PAC_OK && cand >= 0 && c.tuner.best < 0) {
         // every candidate gives the same lists; keep the fastest tetrahedron
         // stage once each has run on this context's work
@@ -357,6 +369,12 @@ int pac_destroy(pac_ctx *ctx) {
             if (ev) cudaEventDestroy(ev);
         cudaStreamDestroy(ctx->c.copy_stream);
     }
+    if (ctx->c.side) {
+        cudaStreamSynchronize(ctx->c.side);
+        cudaStreamDestroy(ctx->c.side);
+    }
+    for (auto &ev : ctx->c.side_ev)
+        if (ev) cudaEventDestroy(ev);
     for (void *p : ctx->c.pinned)
         if (p) cudaFreeHost(p);
     cudaStreamDestroy(ctx->c.stream);

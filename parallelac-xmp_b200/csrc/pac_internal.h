@@ -59,22 +59,21 @@ struct PipelineConfig {
     int formula;    // pac_formula
     int tet_mode;   // pac_tet_mode
     int verbose;
-    uint64_t queue_entries;  // alpha tetrahedra queued per chunk (32 B each)
+    uint64_t queue_entries;  // alpha tetrahedra queued per chunk (8 B each)
     bool exact;              // decision-exact predicates (strict flavour only)
     int slab_rank, slab_world;  // one slab of a partition by cell order (world > 1)
     bool refute;             // early refutation in the tetrahedron enumeration
     bool verify;             // replay every certified insphere decision (debug)
     // launch shapes (the output does not depend on them)
-    int enum_blocks;   // k_tets_enum<.., 1> blocks per SM
-    int heavy_blocks;  // k_tets_enum<.., kMaxW> blocks per SM
+    int enum_blocks;   // k_tets_enum<1> blocks per SM (balls of at most 64 upper neighbours)
+    int heavy_blocks;  // k_tets_enum<2> and <kMaxW> blocks per SM
     int scan_blocks;   // k_tets_scan blocks per SM
-    int unit_rows;     // rows of a ball of more than 64 upper neighbours per work unit
     int scan_claim;    // queue entries a scan warp claims at a time
 };
 
 // Launch shapes the autotuner tries, and its state per context.
 struct LaunchShape {
-    int enum_blocks, heavy_blocks, scan_blocks, unit_rows, scan_claim;
+    int enum_blocks, heavy_blocks, scan_blocks, scan_claim;
 };
 struct Tuner {
     int next = 0;          // next candidate to measure
@@ -120,6 +119,10 @@ struct Ctx {
     // list emitted early crosses PCIe while the later stages compute
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t copy_ev[4]{};
+    // a second stream for kernels that run beside the main one's, and the
+    // events that order it after and before work there (side_stream)
+    cudaStream_t side = nullptr;
+    cudaEvent_t side_ev[2]{};
     // bytes for the alpha-tetrahedron queue, fixed at the context's first
     // pass (a quarter of the memory free then, at most 12 GiB), so that later
     // passes lay out the pool the same way
@@ -138,6 +141,8 @@ int union_measure_device(Ctx &ctx, const double4 *d_balls, uint32_t n, const uin
 // the host address (nullptr when count is 0).  The copy is complete once
 // copies_join's wait has passed on the context's stream.
 int list_to_host_async(Ctx &c, int which, const uint32_t *src, size_t count, uint32_t **dst);
+// Creates the context's side stream and its events on first use.
+int side_stream(Ctx &c);
 // Makes the context's stream wait for every copy started so far.
 int copies_join(Ctx &c);
 

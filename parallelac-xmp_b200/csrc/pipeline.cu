@@ -31,6 +31,7 @@
 #include "certify.cuh"
 #include "exactpred.cuh"
 #include "pac_internal.h"
+#include "pencil.cuh"
 #include "refarith.cuh"
 #include "sos.cuh"
 
@@ -51,7 +52,9 @@ enum Counter {
     C_CAND_E, C_ALPHA_E, C_CAND_T, C_ALPHA_T, C_CAND_Q, C_ALPHA_Q, C_INSPHERE, C_SOS,
     C_OOB, C_SURV, C_PEND, C_MAXDEG, C_SOS_RANGE, C_BADDEG, C_NEXT, C_FILTER, C_FALLBACK,
     C_KILLED, C_KTESTS, C_CERT, C_CERT_BAD,
-    C_NCOUNTERS
+    C_MAXLEN,                 // largest squared alpha-edge length (bits of a binary32)
+    C_CLASS, C_TAKE = C_CLASS + 3,  // balls per enumeration class, and handed out of each
+    C_NCOUNTERS = C_TAKE + 3
 };
 
 struct MolGrid {
@@ -536,6 +539,7 @@ __global__ void __launch_bounds__(256) k_edges(uint64_t n, const float4 *__restr
     uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     unsigned long long cand_acc = 0, alpha_acc = 0;
+    float len2 = 0.f;  // FILL: the longest alpha edge
     Tally tally;
     for (uint64_t p = warp; p < n; p += nwarps) {
         const MolGrid G = grids[mol_of(mol, p)];
@@ -584,7 +588,12 @@ __global__ void __launch_bounds__(256) k_edges(uint64_t n, const float4 *__restr
             uint32_t l = 0;
             if (act) {
                 l = sbeg + (s - (sinc - scnt));
-                pass = dec_edge<V>(A, pac::ld_ball(&at[l]), alpha, tally);
+                const Ball B = pac::ld_ball(&at[l]);
+                pass = dec_edge<V>(A, B, alpha, tally);
+                if (FILL && pass) {
+                    const float x = A.x - B.x, y = A.y - B.y, z = A.z - B.z;
+                    len2 = fmaxf(len2, x * x + y * y + z * z);
+                }
             }
             unsigned m = __ballot_sync(kFull, pass);
             if (FILL && pass) ER[out + kept + __popc(m & ((1u << lane) - 1))] = l;
@@ -595,6 +604,11 @@ __global__ void __launch_bounds__(256) k_edges(uint64_t n, const float4 *__restr
             cand_acc += total;
             alpha_acc += kept;
         }
+    }
+    if (FILL) {
+        const unsigned bits = __reduce_max_sync(kFull, __float_as_uint(len2));
+        if (lane == 0 && bits > (unsigned)*(volatile unsigned long long *)&ctr[C_MAXLEN])
+            atomicMax(&ctr[C_MAXLEN], (unsigned long long)bits);
     }
     if (!FILL) flush_tally<V>(tally, ctr);
     if (!FILL && lane == 0) {
@@ -747,10 +761,9 @@ struct TetArgs {
     const uint64_t *toff; // as-run fill: output offsets per ball
     uint32_t *tets_out;   // as-run fill: sorted-space vertex quadruples
     unsigned long long *ctr;   // the pass's counters, or a chunk's (enumeration)
-    const uint32_t *cellof;    // global cell of each sorted ball
-    int refute;                // enumeration: refute early against the group's best candidate
+    const unsigned long long *maxlen;  // C_MAXLEN of the pass
+    int refute;                // enumeration: refute early against the group's firsts
     int verify;                // scan: replay every certified decision and count disagreements
-    int unit_rows;             // rows of a large ball per enumeration work unit
     int scan_claim;            // queue entries a scan warp claims at a time
 };
 
@@ -891,14 +904,6 @@ __global__ void __launch_bounds__(256) k_tets(TetArgs A) {
     }
 }
 
-// Positions of v2 < v3 < v4 in ball p's upper-neighbour list N (ascending,
-// deg entries), packed a | b << 8 | c << 16 as the survivor lists hold them.
-__device__ __forceinline__ uint32_t key_of(const uint32_t *N, int deg, uint32_t v2, uint32_t v3,
-                                           uint32_t v4) {
-    return (uint32_t)lbound(N, deg, v2) | ((uint32_t)lbound(N, deg, v3) << 8) |
-           ((uint32_t)lbound(N, deg, v4) << 16);
-}
-
 // Records one tetrahedron that passed the orthosphere test (or, pending,
 // one whose window held an exact zero): the survivor list, the per-ball
 // count, and the marks of its four faces in the `faces` matrices.
@@ -907,12 +912,8 @@ __device__ __noinline__ void emit_survivor(const uint64_t *__restrict__ eoff,
                                            const uint64_t *__restrict__ loff, uint64_t *faces,
                                            uint2 *surv, uint64_t surv_cap, uint2 *pend,
                                            uint64_t pend_cap, unsigned long long *ctr,
-                                           uint32_t *tcount, uint32_t p, uint32_t v2, uint32_t v3,
-                                           uint32_t v4, bool pending) {
-    const uint64_t e0 = eoff[p];
-    const int deg = (int)(eoff[p + 1] - e0);
-    const uint32_t *N = ER + e0;
-    const uint32_t key = key_of(N, deg, v2, v3, v4);
+                                           uint32_t *tcount, uint32_t p, uint32_t key, uint32_t v2,
+                                           uint32_t v3, uint32_t v4, bool pending) {
     if (pending) {
         unsigned long long q = atomicAdd(&ctr[C_PEND], 1ull);
         if (q < pend_cap) pend[q] = make_uint2(p, key);
@@ -921,7 +922,7 @@ __device__ __noinline__ void emit_survivor(const uint64_t *__restrict__ eoff,
     unsigned long long q = atomicAdd(&ctr[C_SURV], 1ull);
     if (q < surv_cap) surv[q] = make_uint2(p, key);
     atomicAdd(&tcount[p], 1u);
-    const int W = (deg + 63) >> 6;
+    const int W = (int)((eoff[p + 1] - eoff[p] + 63) >> 6);
     const uint64_t lp = loff[p];
     const int a = key & 0xff, b = (key >> 8) & 0xff, c = (key >> 16) & 0xff;
     mark_face(faces, lp, W, a, b);
@@ -1044,90 +1045,106 @@ constexpr uint64_t kQBlock = 128;
 // (p, v2 = N[a], v3 = N[b], v4 = N[c]), a < b < c, with (p, v2, v3),
 // (p, v2, v4), (p, v3, v4) alpha triangles (bits of p's link rows) and
 // (v2, v3, v4) one too (a bit of v2's link matrix) -- exactly the
-// reference's candidates (AlphaComplexLargeData.cu:350-529).  Per row a the
-// candidate set of every triangle group (a, b) is built bitwise, the pairs
-// (b, c) are written group by group to a per-warp list in shared memory, and
-// the list is evaluated 32 at a time with every lane busy: markRealTets,
-// then an early refutation, then the queue.
+// reference's candidates (AlphaComplexLargeData.cu:350-529).
 //
-// Early refutation.  Within one group the fourth vertices lie in the pencil
-// of spheres orthogonal to the balls p, v2, v3; on either side of the
-// triangle's plane the candidate whose orthosphere comes first along the
-// pencil lies inside the orthosphere of every other candidate on that side.
-// Each lane's tetrahedron is therefore tested against the best candidate
-// of its group and side found so far (a shared-memory minimum over the
-// lanes' orthocentres projected on the triangle normal), with the
-// reference's own arithmetic (orient3d, insphere_w), provided that ball lies
-// in the reference's window of the tetrahedron (surely_in_window).  A violation there is a
-// violation the reference finds: the tetrahedron is dropped.  The rest
-// (a few per cent) go to the queue.
+// Each candidate needs two answers: is it an alpha tetrahedron (counted),
+// and can it be refuted here, by a ball already at hand that violates its
+// orthosphere?  Within one triangle group (a, b) the fourth vertices lie in
+// the pencil of spheres orthogonal to p, v2, v3; on either side of the
+// triangle's plane the one whose orthosphere comes first along the pencil
+// lies inside the orthospheres of all the others, and the two sides' firsts
+// refute each other unless they are in pencil order.  pencil.cuh gives both
+// answers in some twenty operations, each with a certificate that the
+// reference's arithmetic (or, in the exact mode, the exact polynomials) decides
+// alike.  What it cannot certify, and what is not refuted, goes to the queue,
+// and the scan decides it by the general path.
+//
+// What bounds it: instruction issue and shared memory (DRAM is nearly idle).
+// The work of a ball is one list of its alpha triangles, taken 32 at a time
+// by the warps of a block.  A lane sets up one triangle in shared memory; the
+// 32 triangles' candidates are then cut into equal consecutive shares, a lane
+// walking the bits of its share, so every lane is busy and finding a
+// candidate costs a bit scan, not a search.  That first sweep decides the
+// faces and the alpha tests, lists what is left and leaves each side's first
+// candidate; the second tests the list against the firsts (testing against the
+// best so far in one sweep queues twice as many).  A block per ball also keeps
+// small molecules short: a ball's triangles run on 4 to 16 warps instead of one.
+// Measured against one warp per ball or eight rows, markRealTets and a replayed
+// insphere_w per candidate: the pass at 100,008 balls 18.98 -> 13.15 ms, at 211
+// balls 1.52 -> 1.00 ms, the 2.5 M-ball assembly 340 -> 256 ms.
 struct TetQueue {
-    uint4 *vid;    // (v1, v2, v3, v4); v1 = kNoTet marks an unused slot
-    float4 *sph;   // orthosphere centre (x, y, z) and power of v2, as markRealTets gives them
+    uint2 *ent;    // (ball, key): positions a | b << 8 | c << 16 in its list, and flags;
+                   // ball = kNoTet marks an unused slot
     uint64_t cap;
 };
+constexpr uint32_t kAlphaOpen = 1u << 24;  // the alpha test is left to the scan (counted there)
+constexpr uint32_t kRefuted = 1u << 25;    // refuted: the scan only counts it
+constexpr int kRingSteps = 2;              // candidate steps between writes to the queue
 
+// One triangle of a chunk: pencil::Group and what the sweeps leave.  80 bytes
+// apart, so that consecutive records' 16-byte reads meet no bank twice.
+struct GroupRec {
+    float4 nh;       // n, hmin
+    float4 qe;       // Q, ea
+    float4 tk;       // Q~, k
+    float rg;
+    uint32_t ab;     // a | b << 8
+    uint32_t best[2];  // per side: pencil position (24 bits) | c of its first; then c | (refuted) << 8
+    float2 first[2]; // h, g of the firsts
+};
+static_assert(sizeof(GroupRec) == 80, "bank layout");
+
+// KW words per link row: balls of at most 64, 128 or 256 upper neighbours.
 template <int KW>
-struct EnumSmem;
-// balls of at most 64 upper neighbours: one link word per row, all staged
-template <>
-struct EnumSmem<1> {
-    static constexpr int kDeg = 64, kL2Cap = 64, kWarps = 8, kBufs = 2, kLBufs = 2;
-    float4 sb[kWarps][kDeg];      // balls of p's upper neighbours
-    uint64_t sL[kWarps][kDeg];    // p's link rows
-    uint64_t sL2[kWarps][kLBufs][kL2Cap]; // v2's link rows (when they fit), this row and the next
-    uint32_t sN2[kWarps][kBufs][kMaxDeg];// v2's upper neighbours, this row and the next
-    uint64_t sE2[kWarps][kDeg];   // per neighbour v2: its first upper neighbour's index,
-    uint64_t sLo[kWarps][kDeg];   // its link rows' offset,
-    uint16_t sD2[kWarps][kDeg];   // its upper degree
-    uint32_t sN[kWarps][kDeg];    // p's upper neighbours
-    uint16_t smap[kWarps][kDeg];  // position of N[c] in v2's list, 0xffff: absent
-    uint64_t pm[kWarps][32][1];   // the chunk's groups' fourth vertices (bits c)
-    uint8_t gstart[kWarps][32];   // group starting at each slot of a batch
-    uint8_t sBl[kWarps][kDeg];    // the b's of the row, ascending
-    unsigned long long best[kWarps][64];  // per (j, side): orderable key << 32 | c
-    pac::TetGroup grp[kWarps][32];        // markRealTets' products of the chunk's groups
+struct EnumSmem {
+    static constexpr int kDeg = 64 * KW, kTab = KW == 1 ? 1024 : KW == 2 ? 2048 : 8192;
+    static constexpr int kSlots = KW == 1 ? 224 : 256;  // candidates at a time (one group has fewer)
+    static constexpr int kWords = 2 * KW;
+    static constexpr int kGroups = 1024;  // triangles listed at a time (one row has fewer)
+    static constexpr int kWarps = KW == 1 ? 4 : KW == 2 ? 12 : 16;
+    static constexpr int kBlocks = KW == 1 ? 6 : KW == 2 ? 2 : 1;  // per SM
+    float4 rel[kDeg];            // upper neighbours relative to p, and their lifts s
+    pac::pencil::Point pt[kDeg]; // the same in double
+    uint64_t sL[kDeg * KW];      // p's link rows
+    uint64_t e2[kDeg], l2[kDeg]; // per neighbour: its first upper neighbour's index, its link rows
+    GroupRec group[kWarps][33];  // the chunk's triangles, and one past them
+    float2 hg[kWarps][kSlots];   // per listed candidate: h, g
+    uint32_t pm[kWarps][33][kWords];  // per triangle: its fourth vertices (bits c); all ones past the last
+    uint32_t face[kWarps][4][32];     // and its row of v2's link matrix (128 bits)
+    uint32_t ring[kWarps][32 * (kRingSteps + 1)];  // queue entries waiting for a full write
+    uint16_t cand[kWarps][kSlots];  // listed candidates: group | c << 5 | kCand* bits
+    float st[kDeg];              // lifts of the rounded squares
+    uint32_t sN[kDeg];           // upper neighbours
+    uint32_t rowpre[kDeg + 1];   // triangles with fourth vertices before each row
+    uint32_t next, chunk;        // the block's ball, its next chunk
+    uint16_t tri[kGroups];       // p's triangles: a | b << 8
+    pac::pencil::Bounds bounds;  // of the block's ball
+    uint16_t d2[kDeg];           // per neighbour: its upper degree
+    uint8_t tab[kTab];           // positions of p's neighbours by a hash of their index
+    uint8_t map[kDeg][kDeg];     // [a][c]: position of N[c] in the list of N[a] (alpha edges only)
 };
-// larger balls: rows read in place, v2's rows staged when they fit
-template <>
-struct EnumSmem<kMaxW> {
-    static constexpr int kDeg = kMaxDeg, kL2Cap = 256, kWarps = 4, kBufs = 2, kLBufs = 1;
-    float4 sb[kWarps][kDeg];
-    uint64_t sL2[kWarps][kLBufs][kL2Cap];  // this row's only
-    uint32_t sN2[kWarps][kBufs][kMaxDeg];  // this row and the next
-    uint32_t sN[kWarps][kDeg];
-    uint16_t smap[kWarps][kDeg];
-    uint64_t pm[kWarps][32][kMaxW];
-    uint8_t gstart[kWarps][32];
-    uint8_t sBl[kWarps][kDeg];
-    unsigned long long best[kWarps][64];
-    pac::TetGroup grp[kWarps][32];
-};
+// a listed candidate's alpha test is open; |h| >= hmin (and refutation is on)
+constexpr uint32_t kCandOpen = 1u << 13, kCandSure = 1u << 14;
 
-// Per-warp state of the queue reservation.
+// Per-warp state of the queue: the reserved block and the waiting entries.
 struct QRes {
     uint64_t pos, end;  // next free slot of the warp's block, its end
+    int wait;           // entries in the ring
 };
 
-// Appends the lanes with `take` to the queue (warp-uniform call).
-__device__ __forceinline__ void queue_append(const TetQueue &Q, unsigned long long *ctr, QRes &qr,
-                                             bool take, uint4 vid, float4 sph) {
+// Writes the first k <= 32 waiting entries of ball p (warp-uniform call).
+__device__ __forceinline__ void queue_write(const TetQueue &Q, unsigned long long *ctr, QRes &qr,
+                                            uint32_t p, const uint32_t *ring, int k) {
     const int lane = threadIdx.x & 31;
-    const unsigned m = __ballot_sync(kFull, take);
-    if (!m) return;
-    const int k = __popc(m), rank = __popc(m & ((1u << lane) - 1));
     const uint64_t left = qr.end - qr.pos;
     uint64_t nb = 0;
     if ((uint64_t)k > left) {
         if (lane == 0) nb = atomicAdd(&ctr[C_SURV], (unsigned long long)kQBlock);
         nb = __shfl_sync(kFull, nb, 0);
     }
-    if (take) {
-        const uint64_t pos = (uint64_t)rank < left ? qr.pos + rank : nb + (rank - left);
-        if (pos < Q.cap) {
-            Q.vid[pos] = vid;
-            Q.sph[pos] = sph;
-        }
+    if (lane < k) {
+        const uint64_t pos = (uint64_t)lane < left ? qr.pos + lane : nb + (lane - left);
+        if (pos < Q.cap) Q.ent[pos] = make_uint2(p, ring[lane]);
     }
     if ((uint64_t)k > left) {
         qr.pos = nb + (k - left);
@@ -1137,472 +1154,530 @@ __device__ __forceinline__ void queue_append(const TetQueue &Q, unsigned long lo
     }
 }
 
+// Writes the ring's full rows of 32 and moves the rest to its front.
+__device__ __forceinline__ void queue_drain(const TetQueue &Q, unsigned long long *ctr, QRes &qr,
+                                            uint32_t p, uint32_t *ring) {
+    if (qr.wait < 32) return;
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    int at = 0;
+    for (; qr.wait >= 32; at += 32, qr.wait -= 32) queue_write(Q, ctr, qr, p, ring + at, 32);
+    const uint32_t rest = lane < qr.wait ? ring[at + lane] : 0u;
+    __syncwarp();
+    if (lane < qr.wait) ring[lane] = rest;
+}
+
 // Marks the rest of the warp's block unused.
 __device__ __forceinline__ void queue_close(const TetQueue &Q, QRes &qr) {
     const int lane = threadIdx.x & 31;
     for (uint64_t s = qr.pos + lane; s < qr.end; s += 32)
-        if (s < Q.cap) Q.vid[s] = make_uint4(kNoTet, 0, 0, 0);
+        if (s < Q.cap) Q.ent[s] = make_uint2(kNoTet, 0);
     qr.pos = qr.end;
 }
 
-// Asynchronous global -> shared copies (cp.async): the row after the
-// current one is fetched while the current one is worked on.
-__device__ __forceinline__ void cp_async4(void *dst, const void *src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
-// Starts copying row a's v2 (upper neighbours and, when they fit, link
-// rows) into buffer buf of the warp's staging (KW = 1), as one cp.async
-// group of this thread.
-__device__ __forceinline__ void row_fetch(const TetArgs &A, EnumSmem<1> &S, int wib, int a,
-                                          int buf) {
+// The balls of [lo, hi) by class (at most 64, 128, 256 upper neighbours; at
+// least 3): list[class * n ..], counted in ctr[C_CLASS + class].
+__global__ void k_classes(uint64_t lo, uint64_t hi, uint64_t n, const uint64_t *eoff,
+                          uint32_t *list, unsigned long long *ctr) {
+    const uint64_t p = lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    const uint64_t e2 = S.sE2[wib][a];
-    const int deg2 = S.sD2[wib][a];
-    const int W2 = (deg2 + 63) >> 6;
-    for (int k = lane; k < deg2; k += 32) cp_async4(&S.sN2[wib][buf][k], &A.ER[e2 + k]);
-    if (deg2 * W2 <= EnumSmem<1>::kL2Cap) {
-        const uint64_t *L2g = A.link + S.sLo[wib][a];
-        for (int k = lane; k < deg2 * W2; k += 32) cp_async8(&S.sL2[wib][buf][k], &L2g[k]);
+    const int deg = p < hi ? (int)(eoff[p + 1] - eoff[p]) : 0;
+    const int mine = deg < 3 ? -1 : deg <= 64 ? 0 : deg <= 128 ? 1 : 2;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const unsigned m = __ballot_sync(kFull, mine == c);
+        if (!m) continue;
+        unsigned long long b = 0;
+        if (lane == 0) b = atomicAdd(&ctr[C_CLASS + c], (unsigned long long)__popc(m));
+        b = __shfl_sync(kFull, b, 0);
+        if (mine == c) list[c * n + b + __popc(m & ((1u << lane) - 1))] = (uint32_t)p;
     }
-    cp_async_commit();
 }
 
-// A heavy row's v2: where its upper neighbours and link rows start, and
-// how many (KW = kMaxW; the light kernel stages these per ball).
-struct RowSrc {
-    uint64_t e2, loff;
-    int deg2;
-    bool valid;
-};
-__device__ __forceinline__ RowSrc row_src(const TetArgs &A, uint32_t v2) {
-    const uint64_t e2 = A.eoff[v2];
-    return RowSrc{e2, A.loff[v2], (int)(A.eoff[v2 + 1] - e2), true};
-}
-// Starts copying a heavy row's v2 neighbours into buffer buf (one cp.async
-// group of this thread, empty when there is no such row).
-__device__ __forceinline__ void heavy_fetch_n2(const TetArgs &A, EnumSmem<kMaxW> &S, int wib,
-                                               const RowSrc &r, int buf) {
-    const int lane = threadIdx.x & 31;
-    if (r.valid)
-        for (int k = lane; k < r.deg2; k += 32) cp_async4(&S.sN2[wib][buf][k], &A.ER[r.e2 + k]);
-    cp_async_commit();
+// How the enumeration treats its inputs: weights and window centres of the
+// exact mode or of the reference's arithmetic, every certified decision
+// replayed or not (verify mode).
+enum : int { kEnumFloat = 0, kEnumExact = 1, kEnumVerify = 2 };
+
+// Slot of ball x in a table of 2^bits, for attempt t: the neighbours of a ball
+// are a few runs of consecutive indices, which the low bits usually keep apart.
+constexpr int kHashTries = 8;
+__device__ __forceinline__ uint32_t hash_slot(uint32_t x, int t, int bits) {
+    return t == 0 ? x & ((1u << bits) - 1) : (x * (2654435769u * (2u * t + 1u))) >> (32 - bits);
 }
 
-// One row a of ball p: v2 = N[a].  N, sb, sCell hold p's upper neighbours,
-// their balls and cells (shared memory); L its link rows (W words each,
-// shared or global); the rest is per-warp scratch.
-template <int V, int KW>
-__device__ __forceinline__ void tet_row(const TetArgs &A, const TetQueue &Q, EnumSmem<KW> &S,
-                                        const int wib, QRes &qr, uint32_t p, int a, int buf,
-                                        const RowSrc &cur, const RowSrc &nxt, int deg, int W,
-                                        const uint64_t *L, const Ball B1, const MolGrid &G,
-                                        bool refute, unsigned long long &cand_acc,
-                                        unsigned long long &alpha_acc, unsigned long long &kill_acc,
-                                        unsigned long long &ktest_acc, Tally &tally) {
-    constexpr int kL2Cap = EnumSmem<KW>::kL2Cap;
-    const int lane = threadIdx.x & 31;
-    const unsigned lt_mask = (1u << lane) - 1;
-    const uint32_t *N = S.sN[wib];
-    const float4 *sb = S.sb[wib];
-    uint64_t ra[KW];
-    int nb = 0;
-#pragma unroll
-    for (int w = 0; w < KW; w++) {
-        ra[w] = w < W ? L[(uint64_t)a * W + w] : 0ull;
-        nb += __popcll(ra[w]);
-    }
-    if constexpr (KW != 1) {
-        // heavy rows in a pipeline of cp.async groups: this row's
-        // neighbours (issued with the row before), its link rows (now), the
-        // next row's neighbours (after the search below); every path
-        // leaves exactly the next row's group pending
-        const int W2c = (cur.deg2 + 63) >> 6;
-        if (nb >= 2 && cur.deg2 * W2c <= EnumSmem<KW>::kL2Cap)
-            for (int k = lane; k < cur.deg2 * W2c; k += 32)
-                cp_async8(&S.sL2[wib][0][k], &A.link[cur.loff + k]);
-        cp_async_commit();
-        cp_async_wait<1>();  // this row's neighbours
-        __syncwarp();
-        if (nb < 2) {
-            if constexpr (KW == kMaxW) heavy_fetch_n2(A, S, wib, nxt, buf ^ 1);
-            cp_async_wait<1>();
-            return;
-        }
-    } else {
-        if (nb < 2) return;
-    }
-    const uint32_t v2 = N[a];
-    uint32_t *sN2 = S.sN2[wib][buf];
-    uint64_t *sL2 = S.sL2[wib][KW == 1 ? buf : 0];
-    uint16_t *smap = S.smap[wib];
-    uint8_t *sBl = S.sBl[wib];
-    int deg2;
-    const uint64_t *L2g;
-    if constexpr (KW == 1) {
-        // v2's lists were copied into buffer buf by row_fetch
-        deg2 = S.sD2[wib][a];
-        L2g = A.link + S.sLo[wib][a];
-    } else {
-        deg2 = cur.deg2;
-        L2g = A.link + cur.loff;
-    }
-    const int W2 = (deg2 + 63) >> 6;
-    const bool l2s = deg2 * W2 <= kL2Cap;
-    // the b's of the row, ascending
-#pragma unroll
-    for (int w = 0; w < KW; w++) {
-        if (w >= W) break;
-        int before = 0;
-#pragma unroll
-        for (int v = 0; v < KW; v++)
-            if (v < w) before += __popcll(ra[v]);
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const bool bit = (ra[w] >> (32 * h + lane)) & 1ull;
-            const unsigned bm = __ballot_sync(kFull, bit);
-            const int lo = (int)__popcll(ra[w] & ((1ull << (32 * h)) - 1ull)) * (h ? 1 : 0);
-            if (bit) sBl[before + lo + __popc(bm & lt_mask)] = (uint8_t)(w * 64 + 32 * h + lane);
-        }
-    }
-    __syncwarp();
-    // position of N[c] in v2's list, for c > a
-    for (int c = a + 1 + lane; c < deg; c += 32) {
-        const uint32_t x = N[c];
-        int lo2 = 0, n2 = deg2;
-        while (n2 > 0) {
-            const int h = n2 >> 1;
-            if (sN2[lo2 + h] < x) {
-                lo2 += h + 1;
-                n2 -= h + 1;
-            } else {
-                n2 = h;
-            }
-        }
-        smap[c] = (lo2 < deg2 && sN2[lo2] == x) ? (uint16_t)lo2 : (uint16_t)0xffff;
-    }
-    if constexpr (KW == kMaxW) {
-        heavy_fetch_n2(A, S, wib, nxt, buf ^ 1);
-        cp_async_wait<1>();  // this row's link rows
-    }
-    __syncwarp();
-    const float e12x = sb[a].x - B1.x, e12y = sb[a].y - B1.y, e12z = sb[a].z - B1.z;
-    const float4 b2 = sb[a];
-    const Ball B2{b2.x, b2.y, b2.z, b2.w};
-    // groups (a, b) in chunks of 32 b's, lane j owning group j
-    for (int k0 = 0; k0 < nb; k0 += 32) {
-        const int nj = min(32, nb - k0);
-        // lane j: the fourth vertices c > b with the three faces at p
-        // (ra & L[b] & above b)
-        uint64_t pm[KW];
-        if (lane < nj) {
-            const int b = sBl[k0 + lane];
-            const int mb = smap[b];  // 0xffff: (v2, v3) has no alpha edge in v2's list
-            if constexpr (V != pac::kExact) {
-                const float4 b3 = sb[b];
-                S.grp[wib][lane] = pac::tet_group(B1, B2, Ball{b3.x, b3.y, b3.z, b3.w});
-            }
-#pragma unroll
-            for (int w = 0; w < KW; w++)
-                pm[w] = (w < W && mb != 0xffff) ? (ra[w] & L[(uint64_t)b * W + w] & above_mask(b, w))
-                                                : 0ull;
-        } else {
-#pragma unroll
-            for (int w = 0; w < KW; w++) pm[w] = 0ull;
-        }
-        // the pre-candidates (faces at p only); the face (v2, v3, v4) is
-        // checked in the batches below, where every lane is busy
-        int cnt = 0;
-#pragma unroll
-        for (int w = 0; w < KW; w++) cnt += __popcll(pm[w]);
-        int incl = cnt;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const int total = __shfl_sync(kFull, incl, 31);
-        // best-so-far slots of the chunk's groups (j, side)
-        S.best[wib][lane] = ~0ull;
-        S.best[wib][lane + 32] = ~0ull;
-        const int myoff = incl - cnt;
-#pragma unroll
-        for (int w = 0; w < KW; w++) S.pm[wib][lane][w] = pm[w];
-        // the chunk's candidates in group order, 32 per batch: slot t holds
-        // the r-th fourth vertex of group j, t = start(j) + r.  A batch finds
-        // its slots' groups from the mask of the group starts inside it; a
-        // slot before the first start continues the previous batch's last
-        // group.
-        int jcarry = 0;
-        for (int s0 = 0; s0 < total; s0 += 32) {
-            __syncwarp();
-            const int rel = myoff - s0;
-            const bool starts = cnt > 0 && rel >= 0 && rel < 32;
-            if (starts) S.gstart[wib][rel] = (uint8_t)lane;
-            const unsigned M = __reduce_or_sync(kFull, starts ? 1u << rel : 0u);
-            __syncwarp();
-            const unsigned upto = M & (0xffffffffu >> (31 - lane));
-            const int j = upto ? (int)S.gstart[wib][31 - __clz(upto)] : jcarry;
-            jcarry = __shfl_sync(kFull, j, 31);
-            const int r = s0 + lane - __shfl_sync(kFull, myoff, j);
-            const bool act = s0 + lane < total;
-            const int c = act ? select_kw<KW>(S.pm[wib][j], r) : 0;
-            const int b = act ? (int)sBl[k0 + j] : 0;
-            bool face = false;
-            if (act) {  // (v2, v3, v4) an alpha triangle: bit of v2's link
-                const int mb = smap[b], mc = smap[c];
-                if (mc != 0xffff) {
-                    const uint64_t at2 = (uint64_t)mb * W2 + (mc >> 6);
-                    face = ((l2s ? sL2[at2] : __ldg(&L2g[at2])) >> (mc & 63)) & 1ull;
-                }
-            }
-            const unsigned mF = __ballot_sync(kFull, face);
-            if (lane == 0) cand_acc += __popc(mF);
-            bool passA = false, side = false;
-            float4 sphere = make_float4(0.f, 0.f, 0.f, 0.f);
-            float key = 0.f;
-            Ball B3{0.f, 0.f, 0.f, 0.f}, B4{0.f, 0.f, 0.f, 0.f};
-            // markRealTets for every candidate, the alpha tetrahedra being
-            // those with the face (v2, v3, v4): a candidate without it, or
-            // outside alpha, can still refute the others (exact mode: the
-            // alpha tetrahedra only)
-            if (V == pac::kExact ? face : act) {
-                const float4 b3 = sb[b], b4 = sb[c];
-                B3 = Ball{b3.x, b3.y, b3.z, b3.w};
-                B4 = Ball{b4.x, b4.y, b4.z, b4.w};
-                if constexpr (V == pac::kExact)
-                    passA = dec_tet<V>(B1, B2, B3, B4, A.alpha, sphere, tally);
-                else
-                    passA = pac::tet_alpha_g(S.grp[wib][j], B2, B3, B4, A.alpha, sphere) && face;
-                {
-                    // the triangle (p, v2, v3)'s normal; the side of v4
-                    // and the pencil position of the orthocentre
-                    const float e13x = B3.x - B1.x, e13y = B3.y - B1.y, e13z = B3.z - B1.z;
-                    const float nx = e12y * e13z - e12z * e13y;
-                    const float ny = e12z * e13x - e12x * e13z;
-                    const float nz = e12x * e13y - e12y * e13x;
-                    side = nx * (B4.x - B1.x) + ny * (B4.y - B1.y) + nz * (B4.z - B1.z) > 0.f;
-                    key = nx * sphere.x + ny * sphere.y + nz * sphere.z;
-                    if (!side) key = -key;
-                }
-            }
-            const unsigned mA = __ballot_sync(kFull, passA);
-            if (lane == 0) alpha_acc += __popc(mA);
-            bool keep = passA;
-            if constexpr (V != pac::kExact) {
-                // the flat tetrahedra (orthocentre 0, LD:577-580) and
-                // non-finite keys take no part
-                const bool suspect = refute && act && isfinite(key) &&
-                                     !(sphere.x == 0.f && sphere.y == 0.f && sphere.z == 0.f);
-                const bool cand_best = suspect && passA;
-                const int slot = j + (side ? 32 : 0);
-                if (suspect) {
-                    const uint32_t kb = __float_as_uint(key);
-                    const uint32_t ok = (kb & 0x80000000u) ? ~kb : (kb | 0x80000000u);
-                    atomicMin(&S.best[wib][slot], ((unsigned long long)ok << 32) | (uint32_t)c);
-                }
-                __syncwarp();
-                if (cand_best) {
-                    int y = (int)(S.best[wib][slot] & 0xffffffffull);
-                    if (y == c) {
-                        // the best so far of its side: the other side's
-                        // best so far refutes it unless the triangle's two
-                        // sides are in pencil order
-                        const unsigned long long o = S.best[wib][slot ^ 32];
-                        if (o != ~0ull) y = (int)(o & 0xffffffffull);
-                    }
-                    const float4 by = sb[y];
-                    if (y != c && surely_in_window(sphere.x, sphere.y, sphere.z, by.x, by.y, by.z,
-                                                   0.99f * G.step)) {
-                        float pa[3] = {B1.x, B1.y, B1.z}, pb[3] = {B2.x, B2.y, B2.z};
-                        float pc[3] = {B3.x, B3.y, B3.z}, pd[3] = {B4.x, B4.y, B4.z};
-                        float pe[3] = {by.x, by.y, by.z};
-                        const float wa = wt<V>(B1.r), wb = wt<V>(B2.r), wc = wt<V>(B3.r),
-                                    wd = wt<V>(B4.r);
-                        const float ori = dec_orient<V>(pa, pb, pc, pd, wa, wb, wc, wd, tally);
-                        const float res = dec_insphere<V>(pa, pb, pc, pd, pe, wa, wb, wc, wd,
-                                                          wt<V>(by.w), tally);
-                        ktest_acc++;
-                        if (ori < 0 ? (res < 0) : (res > 0)) {
-                            keep = false;
-                            kill_acc++;
-                        }
-                    }
-                }
-            }
-            queue_append(Q, A.ctr, qr, keep,
-                         make_uint4(p, v2, act ? N[b] : 0u, act ? N[c] : 0u), sphere);
-        }
-        __syncwarp();
-    }
-    __syncwarp();
+// Sum over the coordinates of (binary32 square - square); each difference is
+// exact.
+__device__ __forceinline__ float square_rounding(float x, float y, float z) {
+    const float xx = __fmul_rn(x, x), yy = __fmul_rn(y, y), zz = __fmul_rn(z, z);
+    return -(fmaf(x, x, -xx) + fmaf(y, y, -yy) + fmaf(z, z, -zz));
 }
 
-// k_tets_enum: one warp per ball (KW = 1: balls of at most 64 upper
-// neighbours, taken from a counter over the chunk [lo, hi)) or per group of
-// A.unit_rows rows of a larger ball (KW = kMaxW: units from the prefix uoff of
-// k_heavy_rows over [lo, hi)).  The ball's neighbours, their balls and cells
-// (and, for KW = 1, its link rows) are staged in shared memory.
-template <int V, int KW>
-__global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, KW == 1 ? 3 : 4)
-    k_tets_enum(TetArgs A, TetQueue Q, uint64_t lo, uint64_t hi, const uint64_t *uoff) {
+// Verify mode: a certified alpha decision (alpha) and, when y >= 0, a
+// certified refutation by ball y, against the general path; counted in
+// C_CERT (decisions) and C_CERT_BAD (disagreements).
+template <int M>
+__device__ __noinline__ void enum_verify(const TetArgs &A, const MolGrid &G, const float4 b1,
+                                         const float4 b2, const float4 b3, const float4 b4,
+                                         int alpha, const float4 *y) {
+    constexpr int V = (M & kEnumExact) ? pac::kExact : pac::kUpstream;
+    Tally tally;
+    float4 sph;
+    const Ball B1{b1.x, b1.y, b1.z, b1.w}, B2{b2.x, b2.y, b2.z, b2.w}, B3{b3.x, b3.y, b3.z, b3.w},
+        B4{b4.x, b4.y, b4.z, b4.w};
+    const bool mark = dec_tet<V>(B1, B2, B3, B4, A.alpha, sph, tally);
+    if (alpha >= 0) {
+        atomicAdd(&A.ctr[C_CERT], 1ull);
+        if (mark != (alpha == 1)) atomicAdd(&A.ctr[C_CERT_BAD], 1ull);
+    }
+    if (y && mark) {
+        const float pa[3] = {B1.x, B1.y, B1.z}, pb[3] = {B2.x, B2.y, B2.z};
+        const float pc[3] = {B3.x, B3.y, B3.z}, pd[3] = {B4.x, B4.y, B4.z};
+        const float pe[3] = {y->x, y->y, y->z};
+        const float wa = wt<V>(B1.r), wb = wt<V>(B2.r), wc = wt<V>(B3.r), wd = wt<V>(B4.r);
+        const float o = dec_orient<V>(pa, pb, pc, pd, wa, wb, wc, wd, tally);
+        const float r = dec_insphere<V>(pa, pb, pc, pd, pe, wa, wb, wc, wd, wt<V>(y->w), tally);
+        atomicAdd(&A.ctr[C_CERT], 1ull);
+        if (!(o < 0 ? r < 0 : r > 0) ||
+            !surely_in_window(sph.x, sph.y, sph.z, y->x, y->y, y->z, 0.99f * G.step))
+            atomicAdd(&A.ctr[C_CERT_BAD], 1ull);
+    }
+}
+
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Whether ball v lies within reach, per axis, of the orthosphere centre of the
+// candidate z (both relative to p) of a group.
+__device__ __noinline__ bool within_reach(const float4 gA, const float4 gC, const float4 z, float st,
+                                          const float4 v, float reach) {
+    const float h = pac::pencil::height(gA.x, gA.y, gA.z, z.x, z.y, z.z);
+    const float gt = pac::pencil::power(gC.x, gC.y, gC.z, st, z.x, z.y, z.z);
+    return pac::pencil::within_reach(gA.x, gA.y, gA.z, gC.x, gC.y, gC.z, h, gt, v.x, v.y, v.z, reach);
+}
+
+// A block per ball of one class (list, counted in ctr[C_CLASS + cls], taken
+// from ctr[C_TAKE + cls]).
+template <int KW, int M>
+__global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBlocks)
+    k_tets_enum(TetArgs A, TetQueue Q, const uint32_t *list, int cls) {
+    using Smem = EnumSmem<KW>;
+    constexpr int kWarps = Smem::kWarps, kThreads = kWarps * 32, kSlots = Smem::kSlots;
+    constexpr int kTabBits = KW == 1 ? 10 : KW == 2 ? 11 : 13;
+    static_assert(1 << kTabBits == Smem::kTab, "table size");
+#ifdef PAC_CONTRACTED
+    constexpr bool kContracted = !(M & kEnumExact);
+#else
+    constexpr bool kContracted = false;
+#endif
+    // (contracted: half of the squares' rounding, see pencil.cuh)
+    constexpr bool kPerturbed = !(M & kEnumExact);
+    constexpr double kShare = kContracted ? 0.5 : 1.0;
     // more than the 48 KB of static shared memory: dynamic, opted in by
     // enum_smem_optin()
     extern __shared__ __align__(16) unsigned char enum_smem[];
-    EnumSmem<KW> &S = *reinterpret_cast<EnumSmem<KW> *>(enum_smem);
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    unsigned long long cand_acc = 0, alpha_acc = 0, kill_acc = 0, ktest_acc = 0;
-    Tally tally;
-    QRes qr{0, 0};
-    const uint64_t u0 = KW == 1 ? lo : uoff[lo], u1 = KW == 1 ? hi : uoff[hi];
+    Smem &S = *reinterpret_cast<Smem *>(enum_smem);
+    const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
+    const unsigned lt_mask = (1u << lane) - 1;
+    uint32_t cand_acc = 0, open_acc = 0, listed_acc = 0, queued = 0;
+    QRes qr{0, 0, 0};
+    const uint64_t count = A.ctr[C_CLASS + cls];
     while (true) {
-        uint64_t u = 0;
-        if (lane == 0) {
+        // (the previous ball's shared memory is free: every warp passed the
+        // barrier after its last chunk)
+        if (tid == 0) {
             // stop handing out work once the queue has overflowed: the chunk
             // is rerun smaller
-            u = (*(volatile unsigned long long *)&A.ctr[C_SURV] > Q.cap)
-                    ? u1
-                    : u0 + atomicAdd(&A.ctr[C_NEXT], 1ull);
+            unsigned long long u = count;
+            if (!(*(volatile unsigned long long *)&A.ctr[C_SURV] > Q.cap))
+                u = atomicAdd(&A.ctr[C_TAKE + cls], 1ull);
+            S.next = u < count ? list[u] : kNoTet;
+            S.chunk = 0;
         }
-        u = __shfl_sync(kFull, u, 0);
-        if (u >= u1) break;
-        uint64_t p = u;
-        int a0 = 0;
-        if constexpr (KW != 1) {
-            uint64_t pl = lo, ph = hi;  // uoff[pl] <= u < uoff[ph]
-            while (ph - pl > 1) {
-                const uint64_t mid = (pl + ph) >> 1;
-                if (uoff[mid] <= u) pl = mid;
-                else ph = mid;
-            }
-            p = pl;
-            a0 = (int)(u - uoff[p]) * A.unit_rows;
-        }
+        __syncthreads();
+        const uint32_t p = S.next;
+        if (p == kNoTet) break;
         const uint64_t e0 = A.eoff[p];
         const int deg = (int)(A.eoff[p + 1] - e0);
-        if (KW == 1 && (deg < 3 || deg > 64)) continue;  // the heavy kernel takes the larger balls
-        const int W = (deg + 63) >> 6;
-        const uint32_t *Ng = A.ER + e0;
-        const uint64_t *Lg = A.link + A.loff[p];
-        const MolGrid G = A.grids[mol_of(A.mol, p)];
+        const MolGrid &G = A.grids[mol_of(A.mol, p)];
+        const float4 b1 = __ldg(&A.at[p]);
+        const float w1 = __fmul_rn(b1.w, b1.w);  // (its rounding in the exact mode is inside the bounds)
         const bool refute = A.refute && G.gx <= 16384 && G.gy <= 16384 && G.gz <= 16384;
-        for (int c = a0 + lane; c < deg; c += 32) {
-            const uint32_t x = __ldg(&Ng[c]);
-            S.sN[wib][c] = x;
-            S.sb[wib][c] = __ldg(&A.at[x]);
-            if constexpr (KW == 1) {
-                S.sL[wib][c] = Lg[c];
+        if (tid == 0)
+            S.bounds = pac::pencil::bounds(b1.x, b1.y, b1.z, A.alpha,
+                                           __uint_as_float((uint32_t)*A.maxlen), G.wmax, G.step,
+                                           kContracted);
+        // ---- the ball's neighbours, relative to it, and its link rows
+        {
+            const double px = b1.x, py = b1.y, pz = b1.z;
+            const double wp = (M & kEnumExact) ? (double)b1.w * b1.w : (double)w1;
+            const float rp = kPerturbed ? square_rounding(b1.x, b1.y, b1.z) : 0.f;
+            for (int c = tid; c < deg; c += kThreads) {
+                const uint32_t x = __ldg(&A.ER[e0 + c]);
+                const float4 b = __ldg(&A.at[x]);
+                S.sN[c] = x;
+                pac::pencil::Point P;
+                P.x = b.x - px, P.y = b.y - py, P.z = b.z - pz;
+                const double w = (M & kEnumExact) ? (double)b.w * b.w : (double)__fmul_rn(b.w, b.w);
+                P.s = P.x * P.x + P.y * P.y + P.z * P.z - w + wp;
+                P.st = kPerturbed ? P.s + kShare * (square_rounding(b.x, b.y, b.z) - rp) : P.s;
+                S.pt[c] = P;
+                S.rel[c] = make_float4((float)P.x, (float)P.y, (float)P.z, (float)P.s);
+                S.st[c] = (float)P.st;
                 const uint64_t e2 = A.eoff[x];
-                S.sE2[wib][c] = e2;
-                S.sD2[wib][c] = (uint16_t)(A.eoff[x + 1] - e2);
-                S.sLo[wib][c] = A.loff[x];
+                S.e2[c] = e2;
+                S.d2[c] = (uint16_t)(A.eoff[x + 1] - e2);
+                S.l2[c] = A.loff[x];
+                S.tab[hash_slot(x, 0, kTabBits)] = (uint8_t)c;
+            }
+            const int W = (deg + 63) >> 6;
+            const uint64_t *Lg = A.link + A.loff[p];
+            for (int k = tid; k < deg * KW; k += kThreads) {
+                const int a = k / KW, w = k % KW;
+                S.sL[k] = w < W ? Lg[(uint64_t)a * W + w] : 0ull;
             }
         }
-        const Ball B1 = pac::ld_ball(&A.at[p]);
-        __syncwarp();
-        if constexpr (KW == 1) {
-            // the rows with at least two link bits, each one's v2 fetched
-            // while the one before it is worked on
-            const int a1 = deg - 2;
-            uint64_t rows = 0;
+        // (whether some neighbour's rows are wider than a staged face row)
+        bool wide = false;
+        for (int c = tid; c < deg; c += kThreads) wide |= S.d2[c] > 128;
+        wide = __syncthreads_or(wide);
+        // ---- a table without collisions, so that a lookup is one read
+        int tries = 0;
+        while (true) {
+            bool clash = false;
+            for (int c = tid; c < deg; c += kThreads)
+                clash |= S.tab[hash_slot(S.sN[c], tries, kTabBits)] != (uint8_t)c;
+            if (!__syncthreads_or(clash) || ++tries == kHashTries) break;
+            for (int c = tid; c < deg; c += kThreads)
+                S.tab[hash_slot(S.sN[c], tries, kTabBits)] = (uint8_t)c;
+            __syncthreads();
+        }
+        // ---- where each neighbour's neighbours stand in p's list: lanes
+        // over the list of N[a], one lookup each (the last warp also counts
+        // the triangles before each row: its bits but the highest, which has
+        // no fourth vertex above)
+        if (wib == kWarps - 1) {
+            uint32_t base = 0;
+            for (int a0 = 0; a0 < deg; a0 += 32) {
+                const int a = a0 + lane;
+                uint32_t nb = 0;
+                if (a < deg)
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int a = 32 * h + lane;
-                const bool use = a < a1 && __popcll(S.sL[wib][a]) >= 2;
-                rows |= (uint64_t)__ballot_sync(kFull, use) << (32 * h);
+                    for (int w = 0; w < KW; w++) nb += __popcll(S.sL[a * KW + w]);
+                nb -= nb > 0;
+                uint32_t incl = nb;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                if (a < deg) S.rowpre[a] = base + incl - nb;
+                base += __shfl_sync(kFull, incl, 31);
             }
-            int buf = 0;
-            if (rows) row_fetch(A, S, wib, __ffsll((long long)rows) - 1, 0);
-            while (rows) {
-                const int a = __ffsll((long long)rows) - 1;
-                rows &= rows - 1;
-                if (rows) {
-                    row_fetch(A, S, wib, __ffsll((long long)rows) - 1, buf ^ 1);
-                    cp_async_wait<1>();
+            if (lane == 0) S.rowpre[deg] = base;
+        }
+        for (int a = wib; a < deg - 2; a += kWarps) {
+            const uint32_t *N2 = A.ER + S.e2[a];
+            const int deg2 = S.d2[a];
+            for (int k = lane; k < deg2; k += 32) {
+                const uint32_t x = __ldg(&N2[k]);
+                int c;
+                if (tries < kHashTries) {
+                    // a slot no neighbour of p wrote holds anything: the
+                    // comparison settles it
+                    c = S.tab[hash_slot(x, tries, kTabBits)] & (Smem::kDeg - 1);
                 } else {
-                    cp_async_wait<0>();
+                    int hi = deg;
+                    for (c = 0; hi - c > 1;) {
+                        const int mid = (c + hi) >> 1;
+                        if (S.sN[mid] <= x) c = mid;
+                        else hi = mid;
+                    }
                 }
-                __syncwarp();
-                tet_row<V, KW>(A, Q, S, wib, qr, (uint32_t)p, a, buf, RowSrc{}, RowSrc{}, deg, W,
-                               S.sL[wib], B1, G, refute, cand_acc, alpha_acc, kill_acc, ktest_acc,
-                               tally);
-                __syncwarp();
-                buf ^= 1;
+                if (S.sN[c] == x) S.map[a][c] = (uint8_t)k;
             }
-        } else {
-            const int a1 = min(a0 + A.unit_rows, deg - 2);
-            if constexpr (KW == kMaxW) {
-                // each row's v2 neighbours fetched while the row before
-                // is worked on (tet_row keeps the cp.async pipeline)
-                RowSrc cur = a0 < a1 ? row_src(A, S.sN[wib][a0]) : RowSrc{};
-                int buf = 0;
-                heavy_fetch_n2(A, S, wib, cur, buf);
-                for (int a = a0; a < a1; a++) {
-                    const RowSrc nxt = a + 1 < a1 ? row_src(A, S.sN[wib][a + 1]) : RowSrc{};
-                    tet_row<V, KW>(A, Q, S, wib, qr, (uint32_t)p, a, buf, cur, nxt, deg, W, Lg,
-                                   B1, G, refute, cand_acc, alpha_acc, kill_acc, ktest_acc, tally);
-                    cur = nxt;
-                    buf ^= 1;
+        }
+        __syncthreads();
+        const bool slow = S.bounds.reach > 0.f || (M & kEnumVerify);
+        const float kappa = S.bounds.kappa;
+        // ---- the triangles (p, N[a], N[b]): rows [row0, row1) listed at a
+        // time, 32 triangles per chunk
+        for (int row0 = 0, row1; row0 < deg; row0 = row1) {
+        const int listed = (int)S.rowpre[row0];
+        row1 = deg;
+        if (KW > 1 || (int)S.rowpre[deg] > Smem::kGroups) {
+            int lo = row0 + 1, hi = deg;  // the last row whose end fits
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if ((int)S.rowpre[mid] - listed <= Smem::kGroups) lo = mid;
+                else hi = mid - 1;
+            }
+            row1 = lo;
+        }
+        for (int a = row0 + tid; a < row1; a += kThreads) {
+            uint16_t *out = &S.tri[S.rowpre[a] - listed];
+            int left = (int)(S.rowpre[a + 1] - S.rowpre[a]);
+            for (int w = 0; w < 2 * KW && left > 0; w++) {
+                uint32_t bits = ((const uint32_t *)&S.sL[a * KW])[w];
+                for (; bits && left > 0; left--) {
+                    *out++ = (uint16_t)(a | ((w * 32 + __ffs((int)bits) - 1) << 8));
+                    bits &= bits - 1;
                 }
-                cp_async_wait<0>();
+            }
+        }
+        const int ngroups = (int)S.rowpre[row1] - listed;
+        __syncthreads();
+        while (true) {
+            int g0 = 0;
+            if (lane == 0) g0 = (int)atomicAdd(&S.chunk, 32u);
+            g0 = __shfl_sync(kFull, g0, 0);
+            if (g0 >= ngroups) break;
+            // lane: its triangle, and the fourth vertices c > b with the
+            // three faces at p
+            uint64_t pm[KW];
+            int cnt = 0, a = 0, b = 0;
+#pragma unroll
+            for (int w = 0; w < KW; w++) pm[w] = 0ull;
+            if (g0 + lane < ngroups) {
+                const int ab = S.tri[g0 + lane];
+                a = ab & 0xff, b = ab >> 8;
+#pragma unroll
+                for (int w = 0; w < KW; w++) {
+                    pm[w] = S.sL[a * KW + w] & S.sL[b * KW + w] & above_mask(b, w);
+                    cnt += __popcll(pm[w]);
+                }
+            }
+            int incl = cnt;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(kFull, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const int total = __shfl_sync(kFull, incl, 31);
+            if (!total) continue;
+            // the triangles with candidates, side by side in shared memory
+            const unsigned used = __ballot_sync(kFull, cnt > 0);
+            const int r = __popc(used & lt_mask);
+            if (cnt > 0) {
+                const int W2 = (S.d2[a] + 63) >> 6;
+                const uint64_t *row = A.link + S.l2[a] + (uint64_t)S.map[a][b] * W2;
+                const uint64_t f0 = __ldg(&row[0]), f1 = W2 > 1 ? __ldg(&row[1]) : 0ull;
+                const pac::pencil::Group gr = pac::pencil::group(S.bounds, S.pt[a], S.pt[b], w1);
+                GroupRec &R = S.group[wib][r];
+                R.nh = make_float4(gr.nx, gr.ny, gr.nz, gr.hmin);
+                R.qe = make_float4(gr.qx, gr.qy, gr.qz, gr.ea);
+                R.tk = make_float4(gr.tx, gr.ty, gr.tz, gr.k);
+                R.rg = gr.rg;
+                R.ab = (uint32_t)a | ((uint32_t)b << 8);
+                R.best[0] = R.best[1] = 0xffffffffu;
+                S.face[wib][0][r] = (uint32_t)f0;
+                S.face[wib][1][r] = (uint32_t)(f0 >> 32);
+                S.face[wib][2][r] = (uint32_t)f1;
+                S.face[wib][3][r] = (uint32_t)(f1 >> 32);
+#pragma unroll
+                for (int w = 0; w < KW; w++) *(uint64_t *)&S.pm[wib][r][2 * w] = pm[w];
+            }
+            if (lane == 0) {  // ends every walk: lanes past their share read these
+                S.pm[wib][__popc(used)][0] = 0xffffffffu;
+                S.group[wib][__popc(used)].ab = 0;
+            }
+            __syncwarp();
+            // as many whole triangles as the list holds at a time
+            for (int base = 0; base < total;) {
+                const unsigned fits = __ballot_sync(kFull, incl - base <= kSlots);
+                const int end = __shfl_sync(kFull, incl, 31 - __clz((int)fits));
+                const bool mine = cnt > 0 && incl > base && incl <= end;
+                // equal shares: lane takes candidates [start, start + left)
+                const int steps = (end - base + 31) >> 5;
+                const int start = base + lane * steps, left = max(0, min(end - start, steps));
+                int lo = 0;  // first lane whose inclusive count exceeds start
+                for (int o = 16; o; o >>= 1) {
+                    const int v = __shfl_sync(kFull, incl, lo + o - 1);
+                    if (v <= start) lo += o;
+                }
+                const int skip = start - __shfl_sync(kFull, incl - cnt, lo & 31);
+                const uint32_t *words = &S.pm[wib][0][0];
+                // the share's first word, and what it holds of it (a lane
+                // without a share walks along, its results unused)
+                uint32_t k = (uint32_t)__popc(used) * Smem::kWords;
+                uint32_t bits = 0xffffffffu;
+                if (left > 0) {
+                    const uint32_t j = __popc(used & ((1u << lo) - 1));
+                    uint64_t m[KW];
+#pragma unroll
+                    for (int w = 0; w < KW; w++) m[w] = *(const uint64_t *)&S.pm[wib][j][2 * w];
+                    const int c = select_kw<KW>(m, skip);
+                    k = j * Smem::kWords + (c >> 5);
+                    bits = words[k] & (~0u << (c & 31));
+                }
+                base = end;
+                // ---- first sweep: faces, alpha tests, the firsts
+                int n = 0;  // listed
+                for (int s = 0; s < steps; s++) {
+                    const bool act = s < left;
+                    while (!bits) bits = words[++k];
+                    const uint32_t j = k / Smem::kWords;
+                    const uint32_t c = (k % Smem::kWords) * 32 + (uint32_t)__ffs((int)bits) - 1;
+                    bits &= bits - 1;
+                    GroupRec &R = S.group[wib][j];
+                    const uint32_t ab = R.ab;
+                    const uint32_t mc = S.map[ab & 0xff][c];
+                    uint32_t row = S.face[wib][(mc >> 5) & 3][j];
+                    if (wide && act && S.d2[ab & 0xff] > 128)
+                        row = ((const uint32_t *)&A.link[S.l2[ab & 0xff] +
+                                                         (uint64_t)S.map[ab & 0xff][ab >> 8] *
+                                                             ((S.d2[ab & 0xff] + 63) >> 6)])[mc >> 5];
+                    const bool face = act && ((row >> (mc & 31)) & 1u);
+                    const float4 z = S.rel[c], nh = R.nh, qe = R.qe, tk = R.tk;
+                    const float h = pac::pencil::height(nh.x, nh.y, nh.z, z.x, z.y, z.z);
+                    const float q = pac::pencil::power(qe.x, qe.y, qe.z, z.w, z.x, z.y, z.z);
+                    const float gt = kPerturbed
+                                         ? pac::pencil::power(tk.x, tk.y, tk.z, S.st[c], z.x, z.y, z.z)
+                                         : q;
+                    const float a0 = fabsf(h);
+                    const bool sure = a0 >= nh.w;
+                    bool in, out;
+                    pac::pencil::alpha_test(a0, gt, tk.w, qe.w, in, out);
+                    const bool certain = a0 >= kappa * nh.w;
+                    in = in && certain, out = out && certain;
+                    const int i = __float_as_int(q * rcp_approx(a0));
+                    const uint32_t ord = (uint32_t)(i ^ ((i >> 31) | (int)0x80000000));
+                    if (sure && act) atomicMin(&R.best[h > 0.f], (ord & ~0xffu) | c);
+                    const bool live = face && !out, open = live && !in;
+                    cand_acc += face;
+                    open_acc += open;
+                    if constexpr (M & kEnumVerify)
+                        if (face)
+                            enum_verify<M>(A, G, b1, A.at[S.sN[ab & 0xff]], A.at[S.sN[ab >> 8]],
+                                           A.at[S.sN[c]], in ? 1 : out ? 0 : -1, nullptr);
+                    const unsigned m = __ballot_sync(kFull, live);
+                    if (live) {
+                        const int at = n + __popc(m & lt_mask);
+                        S.cand[wib][at] = (uint16_t)(j | (c << 5) | (open ? kCandOpen : 0u) |
+                                                     (sure ? kCandSure : 0u));
+                        S.hg[wib][at] = make_float2(h, q);
+                    }
+                    n += __popc(m);
+                }
+                listed_acc += (uint32_t)n;
+                __syncwarp();
+                // ---- per triangle: its firsts, and whether they refute each other
+                if (mine) {
+                    GroupRec &R = S.group[wib][r];
+                    const float4 nh = R.nh, qe = R.qe;
+                    const uint32_t k0 = R.best[0], k1 = R.best[1];
+                    const int y0 = k0 & 0xff, y1 = k1 & 0xff;
+                    float h0 = 0.f, q0 = 0.f, h1 = 0.f, q1 = 0.f;
+                    if (k0 != 0xffffffffu) {
+                        const float4 z = S.rel[y0];
+                        h0 = pac::pencil::height(nh.x, nh.y, nh.z, z.x, z.y, z.z);
+                        q0 = pac::pencil::power(qe.x, qe.y, qe.z, z.w, z.x, z.y, z.z);
+                    }
+                    if (k1 != 0xffffffffu) {
+                        const float4 z = S.rel[y1];
+                        h1 = pac::pencil::height(nh.x, nh.y, nh.z, z.x, z.y, z.z);
+                        q1 = pac::pencil::power(qe.x, qe.y, qe.z, z.w, z.x, z.y, z.z);
+                    }
+                    // (0 when either side is empty: nothing refuted)
+                    const uint32_t both = pac::pencil::refutes(h0, q0, h1, q1, R.rg) ? 256u : 0u;
+                    R.first[0] = make_float2(h0, q0);
+                    R.first[1] = make_float2(h1, q1);
+                    R.best[0] = (uint32_t)y0 | both;
+                    R.best[1] = (uint32_t)y1 | both;
+                }
+                __syncwarp();
+                // ---- second sweep: refutation; the rest to the queue
+                for (int i0 = 0; i0 < n; i0 += 32 * kRingSteps) {
+#pragma unroll
+                    for (int u = 0; u < kRingSteps; u++) {
+                        const int i = i0 + 32 * u + lane;
+                        bool take = false;
+                        uint32_t key = 0;
+                        if (i < n) {
+                            const uint32_t e = S.cand[wib][i];
+                            const int c = (e >> 5) & 0xff;
+                            const float2 x = S.hg[wib][i];
+                            const GroupRec &R = S.group[wib][e & 31];
+                            const int side = x.x > 0.f;
+                            const uint32_t own = R.best[side];
+                            const float2 y = R.first[side];
+                            bool dead = pac::pencil::refutes(x.x, x.y, y.x, y.y, R.rg);
+                            if (c == (int)(own & 0xff)) dead = own >= 256u;
+                            dead = dead && refute && (e & kCandSure);
+                            if (slow) {
+                                int v = own & 0xff;
+                                if (v == c) v = R.best[side ^ 1] & 0xff;
+                                if (dead && S.bounds.reach > 0.f)
+                                    dead = within_reach(R.nh, R.tk, S.rel[c], S.st[c], S.rel[v],
+                                                        S.bounds.reach);
+                                if constexpr (M & kEnumVerify)
+                                    if (dead)
+                                        enum_verify<M>(A, G, b1, A.at[S.sN[R.ab & 0xff]],
+                                                       A.at[S.sN[R.ab >> 8]], A.at[S.sN[c]],
+                                                       -1, &A.at[S.sN[v]]);
+                            }
+                            take = !dead || (e & kCandOpen);
+                            if (take)
+                                key = R.ab | ((uint32_t)c << 16) |
+                                      (e & kCandOpen ? kAlphaOpen : 0u) | (dead ? kRefuted : 0u);
+                        }
+                        const unsigned m = __ballot_sync(kFull, take);
+                        if (take) S.ring[wib][qr.wait + __popc(m & lt_mask)] = key;
+                        qr.wait += __popc(m);
+                        queued += __popc(m);
+                    }
+                    queue_drain(Q, A.ctr, qr, p, S.ring[wib]);
+                }
                 __syncwarp();
             }
         }
-        __syncwarp();
+        __syncthreads();  // every warp is done with the list
+        if (row1 < deg) {
+            if (tid == 0) S.chunk = 0;
+            __syncthreads();
+        }
+        }
+        if (qr.wait) {
+            __syncwarp();
+            queue_write(Q, A.ctr, qr, p, S.ring[wib], qr.wait);
+            qr.wait = 0;
+            __syncwarp();
+        }
     }
     queue_close(Q, qr);
     // into the chunk's counters: the host adds them to the pass's only when
     // the chunk is accepted (an overflowing chunk is rerun smaller)
-    flush_tally<V>(tally, A.ctr);
+    const unsigned long long cands = warp_sum(cand_acc), open = warp_sum(open_acc);
+    const unsigned long long alphas = listed_acc - open;  // certain ones
     if (lane == 0) {
-        bump(A.ctr, C_CAND_Q, cand_acc);
-        bump(A.ctr, C_ALPHA_Q, alpha_acc);
-    }
-    kill_acc = warp_sum(kill_acc);
-    ktest_acc = warp_sum(ktest_acc);
-    if (lane == 0) {
-        bump(A.ctr, C_KILLED, kill_acc);
-        bump(A.ctr, C_KTESTS, ktest_acc);
+        bump(A.ctr, C_CAND_Q, cands);
+        bump(A.ctr, C_ALPHA_Q, alphas);
+        // every open one is queued, and of the certain ones what is not refuted
+        bump(A.ctr, C_KILLED, alphas - (queued - open));
+        if (A.refute) bump(A.ctr, C_KTESTS, listed_acc);
     }
 }
 
-// Exact-mode tallies and early-refutation counts of an accepted enumeration
+// Early-refutation counts and verify-mode counts of an accepted enumeration
 // chunk into the pass's counters.
 __global__ void k_add_tally(const unsigned long long *chunk, unsigned long long *pass) {
     const int k = threadIdx.x;
     int which = -1;
-    if (k == 0) which = C_FILTER;
-    else if (k == 1) which = C_FALLBACK;
-    else if (k == 2) which = C_SOS_RANGE;
-    else if (k == 3) which = C_KILLED;
-    else if (k == 4) which = C_KTESTS;
+    if (k == 0) which = C_KILLED;
+    else if (k == 1) which = C_KTESTS;
+    else if (k == 2) which = C_CERT;
+    else if (k == 3) which = C_CERT_BAD;
     if (which >= 0 && chunk[which]) pass[which] += chunk[which];
-}
-
-// Work units of the heavy enumeration per ball: ceil((deg - 2) / unit_rows)
-// groups of rows for a ball with more than 64 upper neighbours, 0 for the
-// others.
-__global__ void k_heavy_rows(uint64_t n, const uint64_t *eoff, int unit_rows, uint32_t *rows) {
-    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const uint64_t deg = eoff[p + 1] - eoff[p];
-    rows[p] = deg > 64 ? (uint32_t)((deg - 2 + unit_rows - 1) / unit_rows) : 0u;
 }
 
 constexpr int kScanStep = 4;
 constexpr int kScanRefill = 16;  // idle lanes that trigger a refill
 
 // k_tets_scan: the empty-orthosphere test (checkTetsOrthosphere,
-// AlphaComplexLargeData.cu:606-734) of the queued tetrahedra.  Each lane
+// AlphaComplexLargeData.cu:606-734) of the queued tetrahedra.  An entry's
+// orthosphere comes from markRealTets here (or its exact counterpart), which
+// also settles the alpha tests the enumeration left open.  Each lane
 // owns one tetrahedron at a time and tests kScanStep window balls per step; a warp
 // claims a range of queue entries at a time and a lane takes the next
 // unclaimed one as soon as its own is decided (claims of A.scan_claim
@@ -1617,10 +1692,11 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 2 : 4) k_tets_scan(Tet
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1;
     unsigned long long evals = 0, oob = 0, certd = 0, bad = 0;
+    uint32_t late_alpha = 0, late_killed = 0;  // alpha tests left open by the enumeration
     Tally tally;
     uint64_t head = 0, tail = 0;  // this warp's claimed range (warp-uniform)
     bool have = false, more = true;
-    uint32_t p = 0, v2 = 0, v3 = 0, v4 = 0;
+    uint32_t p = 0, v2 = 0, v3 = 0, v4 = 0, key = 0;
     float ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0, cx = 0, cy = 0, cz = 0, dx = 0, dy = 0,
           dz = 0, wa = 0, wb = 0, wc = 0, wd = 0, orientation = 0;
     pac::cert::Insphere ct{};
@@ -1641,40 +1717,56 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 2 : 4) k_tets_scan(Tet
             head = b;
             tail = min(nq, b + (uint64_t)A.scan_claim);
             if (head >= tail) more = false;
-            for (uint64_t k = head + 4 * lane; k < tail; k += 128) {
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(Q.vid + k));
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(Q.sph + k));
-            }
+            for (uint64_t k = head + 16 * lane; k < tail; k += 512)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(Q.ent + k));
         }
         if (want && head < tail) {
             const int r = __popc(want & lt_mask);
             if (!have && head + r < tail) {
                 const uint64_t idx = head + r;
-                const uint4 vv = Q.vid[idx];
-                if (vv.x != kNoTet) {
-                    const float4 sph = Q.sph[idx];
-                    p = vv.x, v2 = vv.y, v3 = vv.z, v4 = vv.w;
-                    G = A.grids + mol_of(A.mol, p);
+                const uint2 en = Q.ent[idx];
+                if (en.x != kNoTet) {
+                    p = en.x, key = en.y & 0xffffffu;
+                    const uint32_t *N = A.ER + A.eoff[p];
+                    v2 = __ldg(&N[key & 0xff]), v3 = __ldg(&N[(key >> 8) & 0xff]),
+                    v4 = __ldg(&N[key >> 16]);
                     const Ball a1 = pac::ld_ball(&A.at[p]), a2 = pac::ld_ball(&A.at[v2]),
                                a3 = pac::ld_ball(&A.at[v3]), a4 = pac::ld_ball(&A.at[v4]);
-                    ax = a1.x, ay = a1.y, az = a1.z, wa = wt<V>(a1.r);
-                    bx = a2.x, by = a2.y, bz = a2.z, wb = wt<V>(a2.r);
-                    cx = a3.x, cy = a3.y, cz = a3.z, wc = wt<V>(a3.r);
-                    dx = a4.x, dy = a4.y, dz = a4.z, wd = wt<V>(a4.r);
-                    {
+                    float4 sph;
+                    bool mark;
+                    if constexpr (V == pac::kExact)
+                        mark = dec_tet<V>(a1, a2, a3, a4, A.alpha, sph, tally);
+                    else
+                        mark = pac::tet_alpha_g(pac::tet_group(a1, a2, a3), a2, a3, a4, A.alpha, sph);
+                    bool live = true;
+                    if (en.y & kAlphaOpen) {
+                        live = mark && !(en.y & kRefuted);
+                        late_alpha += mark;
+                        late_killed += mark && (en.y & kRefuted);
+                    }
+                    if (live) {
+                        G = A.grids + mol_of(A.mol, p);
+                        ax = a1.x, ay = a1.y, az = a1.z, wa = wt<V>(a1.r);
+                        bx = a2.x, by = a2.y, bz = a2.z, wb = wt<V>(a2.r);
+                        cx = a3.x, cy = a3.y, cz = a3.z, wc = wt<V>(a3.r);
+                        dx = a4.x, dy = a4.y, dz = a4.z, wd = wt<V>(a4.r);
                         const float pa[3] = {ax, ay, az}, pb[3] = {bx, by, bz}, pc[3] = {cx, cy, cz},
                                     pd[3] = {dx, dy, dz};
-                        orientation = dec_orient<V>(pa, pb, pc, pd, wa, wb, wc, wd, tally);
+                        // (exact mode: where the filter's setup accepts it, the
+                        // sign of the binary32 value is the exact one)
+                        orientation = pac::orient3d(pa, pb, pc, pd);
+                        ct = pac::cert::setup(ax, ay, az, a1.r * a1.r, bx, by, bz, a2.r * a2.r, cx, cy,
+                                              cz, a3.r * a3.r, dx, dy, dz, a4.r * a4.r, orientation,
+                                              sph.x, sph.y, sph.z, G->wmax);
+                        if (V == pac::kExact && !ct.ok)
+                            orientation = dec_orient<V>(pa, pb, pc, pd, wa, wb, wc, wd, tally);
+                        const int4 cl = window_cell(*G, sph.x, sph.y, sph.z);
+                        gX = cl.x, gY = cl.y, gZ = cl.z;
+                        q = 0;
+                        zero = false;
+                        window_centre(*G, A.cellbeg, cl, e, end, oob);
+                        have = true;
                     }
-                    if constexpr (V != pac::kExact)
-                        ct = pac::cert::setup(ax, ay, az, wa, bx, by, bz, wb, cx, cy, cz, wc, dx, dy,
-                                              dz, wd, orientation, sph.x, sph.y, sph.z, G->wmax);
-                    const int4 cl = window_cell(*G, sph.x, sph.y, sph.z);
-                    gX = cl.x, gY = cl.y, gZ = cl.z;
-                    q = 0;
-                    zero = false;
-                    window_centre(*G, A.cellbeg, cl, e, end, oob);
-                    have = true;
                 }
             }
             head = min(tail, head + (uint64_t)__popc(want));
@@ -1701,8 +1793,7 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 2 : 4) k_tets_scan(Tet
                 const Ball bb = bq[t];
                 if ((uint32_t)t >= cnt || viol || x == p || x == v2 || x == v3 || x == v4) continue;
                 const float we = wt<V>(bb.r);
-                int dec = -1;
-                if constexpr (V != pac::kExact) dec = pac::cert::test(ct, bb.x, bb.y, bb.z, we);
+                int dec = pac::cert::test(ct, bb.x, bb.y, bb.z, bb.r * bb.r);
                 evals++;
                 if (dec >= 0) certd++;
                 if (dec < 0 || A.verify) {
@@ -1726,7 +1817,7 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 2 : 4) k_tets_scan(Tet
         while (q < kWindowParts && !found) found = window_part(*G, A.cellbeg, gX, gY, gZ, q++, e, end);
         if (!found) {
             emit_survivor(A.eoff, A.ER, A.loff, A.faces, A.surv, A.surv_cap, A.pend, A.pend_cap,
-                          A.ctr, A.tcount, p, v2, v3, v4, zero);
+                          A.ctr, A.tcount, p, key, v2, v3, v4, zero);
             have = false;
         }
     }
@@ -1734,8 +1825,11 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 2 : 4) k_tets_scan(Tet
     oob = warp_sum(oob);
     certd = warp_sum(certd);
     bad = warp_sum(bad);
+    const unsigned long long la = warp_sum(late_alpha), lk = warp_sum(late_killed);
     flush_tally<V>(tally, A.ctr);
     if (lane == 0) {
+        bump(A.ctr, C_ALPHA_Q, la);
+        bump(A.ctr, C_KILLED, lk);
         bump(A.ctr, C_INSPHERE, evals);
         bump(A.ctr, C_OOB, oob);
         bump(A.ctr, C_CERT, certd);
@@ -2226,15 +2320,55 @@ __global__ void k_mol_rows(uint32_t n_mol, const uint64_t *ball_off, uint64_t n,
 // ------------------------------------------------------------------ host
 // The enumeration kernels' shared memory exceeds the static 48 KB: allow it
 // (once per device and flavour; the attribute belongs to the kernel).
-template <int V>
+template <int M>
 static int enum_smem_optin(pac::Ctx &ctx) {
     static bool done[64] = {};
     if (ctx.device >= 0 && ctx.device < 64 && done[ctx.device]) return PAC_OK;
-    CK(cudaFuncSetAttribute(k_tets_enum<V, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CK(cudaFuncSetAttribute(k_tets_enum<1, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)sizeof(EnumSmem<1>)));
-    CK(cudaFuncSetAttribute(k_tets_enum<V, kMaxW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CK(cudaFuncSetAttribute(k_tets_enum<2, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)sizeof(EnumSmem<2>)));
+    CK(cudaFuncSetAttribute(k_tets_enum<kMaxW, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)sizeof(EnumSmem<kMaxW>)));
     if (ctx.device >= 0 && ctx.device < 64) done[ctx.device] = true;
+    return PAC_OK;
+}
+
+// The enumeration of the balls [lo, hi): their classes, then one launch per
+// class that the pass's largest degree can reach, the longest blocks first.
+template <int M>
+static int enumerate(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const TetArgs &A,
+                     const TetQueue &Q, uint64_t lo, uint64_t hi, uint32_t *list, uint64_t maxdeg) {
+    cudaStream_t s = ctx.stream;
+    int rc = enum_smem_optin<M>(ctx);
+    if (rc) return rc;
+    const uint64_t balls = hi - lo;
+    k_classes<<<(unsigned)((balls + 255) / 256), 256, 0, s>>>(lo, hi, A.n, A.eoff, list, A.ctr);
+    LAUNCH_CHECK(ctx);
+    const unsigned light = (unsigned)std::min<uint64_t>(balls, 148u * (unsigned)std::max(1, cfg.enum_blocks));
+    const unsigned heavy = (unsigned)std::min<uint64_t>(balls, 148u * (unsigned)std::max(1, cfg.heavy_blocks));
+    // the few balls of the largest class take long one by one: beside the rest
+    const bool aside = maxdeg > 128;
+    if (aside) {
+        rc = pac::side_stream(ctx);
+        if (rc) return rc;
+        CK(cudaEventRecord(ctx.side_ev[0], s));
+        CK(cudaStreamWaitEvent(ctx.side, ctx.side_ev[0], 0));
+        k_tets_enum<kMaxW, M><<<(unsigned)std::min<uint64_t>(heavy, 148), EnumSmem<kMaxW>::kWarps * 32,
+                                sizeof(EnumSmem<kMaxW>), ctx.side>>>(A, Q, list + 2 * A.n, 2);
+        LAUNCH_CHECK(ctx);
+        CK(cudaEventRecord(ctx.side_ev[1], ctx.side));
+    }
+    if (maxdeg > 64) {
+        k_tets_enum<2, M><<<heavy, EnumSmem<2>::kWarps * 32, sizeof(EnumSmem<2>), s>>>(
+            A, Q, list + A.n, 1);
+        LAUNCH_CHECK(ctx);
+    }
+    if (maxdeg >= 3) {
+        k_tets_enum<1, M><<<light, EnumSmem<1>::kWarps * 32, sizeof(EnumSmem<1>), s>>>(A, Q, list, 0);
+        LAUNCH_CHECK(ctx);
+    }
+    if (aside) CK(cudaStreamWaitEvent(s, ctx.side_ev[1], 0));
     return PAC_OK;
 }
 
@@ -2447,14 +2581,15 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
     T.grids = grids;
     T.alpha = in.alpha;
     T.ctr = ctr;
-    T.cellof = cellof;
+    T.maxlen = ctr + C_MAXLEN;
     T.refute = cfg.refute ? 1 : 0;
     T.verify = cfg.verify ? 1 : 0;
-    T.unit_rows = std::max(1, cfg.unit_rows);
     T.scan_claim = std::max(32, cfg.scan_claim);
     T.tcount = ar.alloc_n<uint32_t>(n);
     uint64_t *toff = ar.alloc_n<uint64_t>(n + 1);
     if (!T.tcount || !toff) return PAC_ERR_OOM;
+    // the enumeration's counts; the scan adds what was left open to it
+    unsigned long long cand_total = 0, alpha_total = 0;
     uint64_t nQ = 0;      // tetrahedra output
     uint64_t nQ_all = 0;  // survivors, a slab's halo included
     uint32_t *tets_sorted = nullptr;
@@ -2477,8 +2612,7 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         // queue of alpha tetrahedra in HBM, processed in chunks of balls
         const uint64_t qcap = std::max<uint64_t>(1 << 16, cfg.queue_entries);
         TetQueue Q;
-        Q.vid = ar.alloc_n<uint4>(qcap);
-        Q.sph = ar.alloc_n<float4>(qcap);
+        Q.ent = ar.alloc_n<uint2>(qcap);
         Q.cap = qcap;
         uint64_t scap = std::max<uint64_t>(1024, 16 * n);
         T.surv = ar.alloc_n<uint2>(scap);
@@ -2487,26 +2621,12 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         T.pend_cap = scap / 4 + 1024;
         unsigned long long *claim = ar.alloc_n<unsigned long long>(1);
         unsigned long long *ctrA = ar.alloc_n<unsigned long long>(C_NCOUNTERS);
-        if (!Q.vid || !Q.sph || !T.surv || !T.pend || !claim || !ctrA) return PAC_ERR_OOM;
+        uint32_t *classes = ar.alloc_n<uint32_t>(3 * n);  // the enumeration's classes of balls
+        if (!Q.ent || !classes || !T.surv || !T.pend || !claim || !ctrA) return PAC_ERR_OOM;
         CK(cudaMemsetAsync(ctr + C_SURV, 0, 2 * sizeof(unsigned long long), s));
         CK(cudaMemsetAsync(ctr + C_INSPHERE, 0, sizeof(unsigned long long), s));
         CK(cudaMemsetAsync(faces, 0, sizeof(uint64_t) * (nL ? nL : 1), s));
         CK(cudaMemsetAsync(T.tcount, 0, sizeof(uint32_t) * n, s));
-        // work units of the balls with more than 64 upper neighbours
-        uint32_t *hrows = ar.alloc_n<uint32_t>(n);
-        uint64_t *uoff = ar.alloc_n<uint64_t>(n + 1);
-        if (!hrows || !uoff) return PAC_ERR_OOM;
-        uint64_t heavy_units = 0;
-        if (maxdeg > 64) {
-            k_heavy_rows<<<blocks_for(n, 256), 256, 0, s>>>(n, eoff, T.unit_rows, hrows);
-            LAUNCH_CHECK(ctx);
-            rc = exclusive_scan(ctx, hrows, n, uoff);
-            if (rc) return rc;
-            CK(cudaMemcpyAsync(&heavy_units, uoff + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-        }
-        rc = enum_smem_optin<V>(ctx);
-        if (rc) return rc;
         // the empty-orthosphere test's share of the stage: ev[14], ev[15]
         // around each scan, read once the stream has passed them
         double ortho_ms = 0.0;
@@ -2517,7 +2637,6 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
             if (cudaEventElapsedTime(&f, ctx.ev[14], ctx.ev[15]) == cudaSuccess) ortho_ms += f;
             ortho_pending = false;
         };
-        unsigned long long cand_total = 0, alpha_total = 0;
         uint64_t lo = work_lo, chunk = n;
         {
             // first chunk: the whole range when its queue demand (a few
@@ -2527,32 +2646,26 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
             unsigned long long atri = 0;
             CK(cudaMemcpyAsync(&atri, ctr + C_ALPHA_T, sizeof(atri), cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));
+            // (about 0.5 entries per alpha triangle; 5 without refutation)
             const double span = (double)(own_hi - work_lo), share = span / (double)std::max<uint64_t>(1, n);
-            if (2.0 * (double)atri * share > 0.85 * (double)qcap)
+            if ((cfg.refute ? 1.0 : 8.0) * (double)atri * share > 0.85 * (double)qcap)
                 chunk = std::max<uint64_t>(1, (uint64_t)(span / 32.0));
         }
         // verbose: per-chunk enumeration and scan times
+        unsigned long long late_before = 0;
         cudaEvent_t vev[3] = {nullptr, nullptr, nullptr};
         if (cfg.verbose)
             for (auto &e : vev) CK(cudaEventCreate(&e));
-        const unsigned enum_blocks = 148u * (unsigned)std::max(1, cfg.enum_blocks);
-        const unsigned heavy_blocks = 148u * (unsigned)std::max(1, cfg.heavy_blocks);
         while (lo < own_hi) {
             const uint64_t hi = std::min<uint64_t>(own_hi, lo + chunk);
             TetArgs TA = T;
             TA.ctr = ctrA;
             if (cfg.verbose) CK(cudaEventRecord(vev[0], s));
             CK(cudaMemsetAsync(ctrA, 0, sizeof(unsigned long long) * C_NCOUNTERS, s));
-            k_tets_enum<V, 1><<<(unsigned)std::min<uint64_t>(enum_blocks, (hi - lo + 7) / 8),
-                                EnumSmem<1>::kWarps * 32, sizeof(EnumSmem<1>), s>>>(TA, Q, lo, hi,
-                                                                                   nullptr);
-            LAUNCH_CHECK(ctx);
-            if (heavy_units) {  // balls with more than 64 upper neighbours, by rows
-                CK(cudaMemsetAsync(ctrA + C_NEXT, 0, sizeof(unsigned long long), s));
-                k_tets_enum<V, kMaxW><<<heavy_blocks, EnumSmem<kMaxW>::kWarps * 32,
-                                        sizeof(EnumSmem<kMaxW>), s>>>(TA, Q, lo, hi, uoff);
-                LAUNCH_CHECK(ctx);
-            }
+            constexpr int M = V == pac::kExact ? kEnumExact : kEnumFloat;
+            rc = cfg.verify ? enumerate<M | kEnumVerify>(ctx, cfg, TA, Q, lo, hi, classes, maxdeg)
+                            : enumerate<M>(ctx, cfg, TA, Q, lo, hi, classes, maxdeg);
+            if (rc) return rc;
             if (cfg.verbose) CK(cudaEventRecord(vev[1], s));
             unsigned long long ha[C_NCOUNTERS], used[2];
             CK(cudaMemcpyAsync(ha, ctrA, sizeof(ha), cudaMemcpyDeviceToHost, s));
@@ -2591,7 +2704,7 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
             }
             cand_total += ha[C_CAND_Q];
             alpha_total += ha[C_ALPHA_Q];
-            if (ha[C_FILTER] || ha[C_FALLBACK] || ha[C_SOS_RANGE] || ha[C_KILLED] || ha[C_KTESTS]) {
+            if (ha[C_KILLED] || ha[C_KTESTS] || ha[C_CERT]) {
                 k_add_tally<<<1, 32, 0, s>>>(ctrA, ctr);
                 LAUNCH_CHECK(ctx);
             }
@@ -2605,15 +2718,18 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
             }
             if (cfg.verbose) {
                 float me = 0.f, ms = 0.f;
+                unsigned long long late = 0;  // alpha tests that the scan settled
                 CK(cudaEventRecord(vev[2], s));
-                CK(cudaEventSynchronize(vev[2]));
+                CK(cudaMemcpyAsync(&late, ctr + C_ALPHA_Q, sizeof(late), cudaMemcpyDeviceToHost, s));
+                CK(cudaStreamSynchronize(s));
                 CK(cudaEventElapsedTime(&me, vev[0], vev[1]));
                 CK(cudaEventElapsedTime(&ms, vev[1], vev[2]));
                 std::fprintf(stderr,
                              "[pac] tetrahedra of balls [%llu, %llu): %llu candidates, %llu alpha, "
                              "%llu refuted early, %llu queued; enumeration %.3f ms, scan %.3f ms\n",
                              (unsigned long long)lo, (unsigned long long)hi, ha[C_CAND_Q],
-                             ha[C_ALPHA_Q], ha[C_KILLED], queued, me, ms);
+                             ha[C_ALPHA_Q] + late - late_before, ha[C_KILLED], queued, me, ms);
+                late_before = late;
             }
             // next chunk sized from this one's queue fill
             if (queued)
@@ -2625,10 +2741,6 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         }
         if (cfg.verbose)
             for (auto &e : vev) cudaEventDestroy(e);
-        {
-            unsigned long long cq[2] = {cand_total, alpha_total};
-            CK(cudaMemcpyAsync(ctr + C_CAND_Q, cq, sizeof(cq), cudaMemcpyHostToDevice, s));
-        }
         unsigned long long sp[2];
         CK(cudaMemcpyAsync(sp, ctr + C_SURV, sizeof(sp), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
@@ -2780,6 +2892,8 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
     unsigned long long hc[C_NCOUNTERS];
     CK(cudaMemcpyAsync(hc, ctr, sizeof(hc), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    hc[C_CAND_Q] += cand_total;
+    hc[C_ALPHA_Q] += alpha_total;
     if (hc[C_SOS_RANGE])
         return pac::set_error(PAC_ERR_EXACT_RANGE,
                               "coordinate range too wide for the exact SoS integers");
