@@ -9,13 +9,19 @@
 // mode does not reproduce those flips, it answers the questions exactly.
 // The candidate sets and the 27-cell windows stay the reference's.
 //
-// Cascade.  Each polynomial is first evaluated in FP64 with a running bound
-// on its absolute error (every operation adds |result| * 2^-53 and products
-// propagate their operands' bounds).  If |value| exceeds the bound the sign
-// is certain.  Otherwise the polynomial is evaluated again in 640-bit
-// two's-complement integers, after writing every input as an integer
-// multiple of one power of two chosen per call; that path is counted
-// (pac_stats.exact_fallbacks).
+// Cascade.  Each polynomial is first evaluated in plain FP64 against a bound
+// from the inputs' extent: no path of any of them has more than 40 roundings
+// (differences and squared radii included), so the error is below
+// 40 * 2^-53 (1 + 2^-40) times the value over operand magnitudes.  Where that
+// cannot tell, it is evaluated in FP64 with a running bound on its absolute
+// error (every operation adds |result| * 2^-53 and products propagate their
+// operands' bounds).  Otherwise the polynomial is evaluated again in
+// two's-complement integers of up to 640 bits, after writing every input as an
+// integer multiple of one power of two chosen per call; that path is counted
+// (pac_stats.exact_fallbacks).  The plain evaluation costs a quarter of the
+// running bound and decides all but near-ties; the running one is kept out of
+// line, its two values per operand spilled every caller (the orthosphere
+// scan of 25,000 lattice-snapped balls 16.8 ms with it in line).
 //
 // Polynomials, with u = p2 - p1, v = p3 - p1, s = p4 - p1, n = u x v and
 // B_k = |p_k - p1|^2 + w1 - w_k (twice the offset of the radical plane of
@@ -75,21 +81,25 @@ __device__ __forceinline__ int ev_sign(const EV a) {
 }
 
 // ------------------------------------------------------------------ integers
+template <int L>
 struct BI {
-    BigInt b;
+    BigInt<L> b;
 };
-__device__ __forceinline__ BI operator+(const BI &a, const BI &b) {
-    BI r;
+template <int L>
+__device__ __forceinline__ BI<L> operator+(const BI<L> &a, const BI<L> &b) {
+    BI<L> r;
     bi_add(r.b, a.b, b.b);
     return r;
 }
-__device__ __forceinline__ BI operator-(const BI &a, const BI &b) {
-    BI r;
+template <int L>
+__device__ __forceinline__ BI<L> operator-(const BI<L> &a, const BI<L> &b) {
+    BI<L> r;
     bi_sub(r.b, a.b, b.b);
     return r;
 }
-__device__ __forceinline__ BI operator*(const BI &a, const BI &b) {
-    BI r;
+template <int L>
+__device__ __forceinline__ BI<L> operator*(const BI<L> &a, const BI<L> &b) {
+    BI<L> r;
     bi_mul(r.b, a.b, b.b);
     return r;
 }
@@ -124,10 +134,16 @@ __device__ __forceinline__ V3<R> add3(const V3<R> &a, const V3<R> &b) {
     return V3<R>{a.x + b.x, a.y + b.y, a.z + b.z};
 }
 
-// Each functor maps points p[0..] (and alpha, and for the attachment tests
+// Each functor (of weighted degree kDegree: coordinates 1, weights and alpha 2)
+// with magnitude(M, B, wa) bounding the polynomial's value over operand
+// magnitudes when coordinates differ by at most M, |B_k| and the lifts are at
+// most B and |w + alpha| at most wa: a component of u is at most M, a dot product
+// 3 M^2, a component of u x v 2 M^2, |n|^2 12 M^4, det(u, v, s) 6 M^3)
+// maps points p[0..] (and alpha, and for the attachment tests
 // the extra ball q = p[last]) to a polynomial whose sign is the decision.
 struct FEdge {  // >= 0: alpha edge (given |u| > 0)
-    static constexpr int kPts = 2;
+    static constexpr int kPts = 2, kDegree = 4;
+    static __device__ float magnitude(float M, float B, float wa) { return 12.f * M * M * wa + B * B; }
     template <class R>
     __device__ R operator()(const P4<R> *p, const R &a) const {
         const V3<R> u = dif(p[1], p[0]);
@@ -138,7 +154,8 @@ struct FEdge {  // >= 0: alpha edge (given |u| > 0)
     }
 };
 struct FNormal2 {  // |n|^2 of a triangle: 0 iff collinear
-    static constexpr int kPts = 3;
+    static constexpr int kPts = 3, kDegree = 4;
+    static __device__ float magnitude(float M, float, float) { return 12.f * M * M * M * M; }
     template <class R>
     __device__ R operator()(const P4<R> *p, const R &) const {
         const V3<R> n = cross(dif(p[1], p[0]), dif(p[2], p[0]));
@@ -146,7 +163,8 @@ struct FNormal2 {  // |n|^2 of a triangle: 0 iff collinear
     }
 };
 struct FTri {  // >= 0: alpha triangle (given n != 0)
-    static constexpr int kPts = 3;
+    static constexpr int kPts = 3, kDegree = 6;
+    static __device__ float magnitude(float M, float B, float wa) { return 48.f * M * M * M * M * wa + 12.f * M * M * B * B; }
     template <class R>
     __device__ R operator()(const P4<R> *p, const R &a) const {
         const V3<R> u = dif(p[1], p[0]), v = dif(p[2], p[0]);
@@ -160,14 +178,16 @@ struct FTri {  // >= 0: alpha triangle (given n != 0)
     }
 };
 struct FDet {  // det(u, v, s) of a tetrahedron
-    static constexpr int kPts = 4;
+    static constexpr int kPts = 4, kDegree = 3;
+    static __device__ float magnitude(float M, float, float) { return 6.f * M * M * M; }
     template <class R>
     __device__ R operator()(const P4<R> *p, const R &) const {
         return dot(dif(p[1], p[0]), cross(dif(p[2], p[0]), dif(p[3], p[0])));
     }
 };
 struct FTet {  // >= 0: alpha tetrahedron (given det != 0)
-    static constexpr int kPts = 4;
+    static constexpr int kPts = 4, kDegree = 8;
+    static __device__ float magnitude(float M, float B, float wa) { return 144.f * M * M * M * M * M * M * wa + 108.f * M * M * M * M * B * B; }
     template <class R>
     __device__ R operator()(const P4<R> *p, const R &a) const {
         const V3<R> u = dif(p[1], p[0]), v = dif(p[2], p[0]), s = dif(p[3], p[0]);
@@ -182,7 +202,8 @@ struct FTet {  // >= 0: alpha tetrahedron (given det != 0)
     }
 };
 struct FEdgeAttach {  // <= 0: ball p[2] attaches edge (p[0], p[1])
-    static constexpr int kPts = 3;
+    static constexpr int kPts = 3, kDegree = 4;
+    static __device__ float magnitude(float M, float B, float) { return 6.f * B * M * M; }
     template <class R>
     __device__ R operator()(const P4<R> *p, const R &) const {
         const V3<R> u = dif(p[1], p[0]), q = dif(p[2], p[0]);
@@ -192,7 +213,8 @@ struct FEdgeAttach {  // <= 0: ball p[2] attaches edge (p[0], p[1])
     }
 };
 struct FTriAttach {  // <= 0: ball p[3] attaches triangle (p[0], p[1], p[2])
-    static constexpr int kPts = 4;
+    static constexpr int kPts = 4, kDegree = 6;
+    static __device__ float magnitude(float M, float B, float) { return 36.f * B * M * M * M * M; }
     template <class R>
     __device__ R operator()(const P4<R> *p, const R &) const {
         const V3<R> u = dif(p[1], p[0]), v = dif(p[2], p[0]), q = dif(p[3], p[0]);
@@ -203,7 +225,8 @@ struct FTriAttach {  // <= 0: ball p[3] attaches triangle (p[0], p[1], p[2])
     }
 };
 struct FOrient {  // orient3d(pa, pb, pc, pd): rows pa - pd, pb - pd, pc - pd
-    static constexpr int kPts = 4;
+    static constexpr int kPts = 4, kDegree = 3;
+    static __device__ float magnitude(float M, float, float) { return 6.f * M * M * M; }
     template <class R>
     __device__ R operator()(const P4<R> *p, const R &) const {
         const V3<R> a = dif(p[0], p[3]), b = dif(p[1], p[3]), c = dif(p[2], p[3]);
@@ -211,7 +234,8 @@ struct FOrient {  // orient3d(pa, pb, pc, pd): rows pa - pd, pb - pd, pc - pd
     }
 };
 struct FInsphere {  // insphere_w(pa, pb, pc, pd, pe) of PRED:4250-4367
-    static constexpr int kPts = 5;
+    static constexpr int kPts = 5, kDegree = 5;
+    static __device__ float magnitude(float M, float B, float) { return 24.f * B * M * M * M; }
     template <class R>
     __device__ R operator()(const P4<R> *p, const R &) const {
         V3<R> d[4];
@@ -246,10 +270,28 @@ __device__ __forceinline__ bool fexp(float f, int &lo, int &hi) {
     return true;
 }
 
-// Exact sign by integers.  *range is set when the inputs span more bits
-// than the 640-bit integers hold for a polynomial of weighted degree 8.
+// Sign of f over integers of L limbs, every input a multiple of 2^E.
+template <int L, class F, int N>
+__device__ __noinline__ int integer_sign(const F f, const Ball (&b)[N], float alpha, int E) {
+    P4<BI<L>> p[N];
+    for (int i = 0; i < N; i++) {
+        bi_from_float(p[i].x.b, b[i].x, E);
+        bi_from_float(p[i].y.b, b[i].y, E);
+        bi_from_float(p[i].z.b, b[i].z, E);
+        BI<L> r;
+        bi_from_float(r.b, b[i].r, E);
+        p[i].w = r * r;
+    }
+    BI<L> a;
+    bi_from_float(a.b, alpha, 2 * E);
+    return bi_sign(f(p, a).b);
+}
+
+// Exact sign by integers, as short as the polynomial's degree and the inputs'
+// range allow.  *range is set when the inputs span more bits than the widest
+// integers hold for a polynomial of weighted degree 8 (whatever f's degree).
 template <class F, int N>
-__device__ __noinline__ int exact_sign(const F f, const Ball (&b)[N], float alpha, int *range) {
+__device__ __forceinline__ int exact_sign(const F f, const Ball (&b)[N], float alpha, int *range) {
     int E = 0, H = -1000, lo, hi;
     for (int i = 0; i < N; i++) {
         const float c[4] = {b[i].x, b[i].y, b[i].z, b[i].r};
@@ -267,18 +309,9 @@ __device__ __noinline__ int exact_sign(const F f, const Ball (&b)[N], float alph
         *range = 1;
         return 0;
     }
-    P4<BI> p[N];
-    for (int i = 0; i < N; i++) {
-        bi_from_float(p[i].x.b, b[i].x, E);
-        bi_from_float(p[i].y.b, b[i].y, E);
-        bi_from_float(p[i].z.b, b[i].z, E);
-        BI r;
-        bi_from_float(r.b, b[i].r, E);
-        p[i].w = r * r;
-    }
-    BI a;
-    bi_from_float(a.b, alpha, 2 * E);
-    return bi_sign(f(p, a).b);
+    if (F::kDegree * (H - E) + 24 <= kLimbsShort * 32 - 1)
+        return integer_sign<kLimbsShort>(f, b, alpha, E);
+    return integer_sign<kLimbs>(f, b, alpha, E);
 }
 
 // Per-thread counts of one kernel: filtered decisions, integer
@@ -289,17 +322,56 @@ struct Tally {
     int range = 0;
 };
 
-// The cascade: FP64 filter, integers when it cannot decide.
+// The running-bound filter alone: 0 when it cannot decide.
 template <class F, int N>
-__device__ __forceinline__ int sign_of(const F f, const Ball (&b)[N], float alpha, Tally &t) {
+__device__ __noinline__ int running_sign(const F f, const Ball (&b)[N], float alpha) {
     P4<EV> p[N];
 #pragma unroll
     for (int i = 0; i < N; i++) {
         const EV r = ev(b[i].r);
         p[i] = P4<EV>{ev(b[i].x), ev(b[i].y), ev(b[i].z), r * r};
     }
+    return ev_sign(f(p, ev(alpha)));
+}
+
+// The plain FP64 evaluation against the bound from the inputs' extent.
+template <class F, int N>
+__device__ __forceinline__ int plain_sign(const F f, const Ball (&b)[N], float alpha) {
+    P4<double> p[N];
+    float lo[3] = {b[0].x, b[0].y, b[0].z}, hi[3] = {b[0].x, b[0].y, b[0].z}, rm = fabsf(b[0].r);
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const double r = b[i].r;
+        p[i] = P4<double>{b[i].x, b[i].y, b[i].z, r * r};
+        lo[0] = fminf(lo[0], b[i].x), hi[0] = fmaxf(hi[0], b[i].x);
+        lo[1] = fminf(lo[1], b[i].y), hi[1] = fmaxf(hi[1], b[i].y);
+        lo[2] = fminf(lo[2], b[i].z), hi[2] = fmaxf(hi[2], b[i].z);
+        rm = fmaxf(rm, fabsf(b[i].r));
+    }
+    const float M = fmaxf(hi[0] - lo[0], fmaxf(hi[1] - lo[1], hi[2] - lo[2])) * 1.00001f;
+    const float W = rm * rm * 1.00001f;
+    // 4.6e-15 > 40 * 2^-53; the factors cover the binary32 rounding here, the
+    // last term results below the normal range
+    const float bound = 4.6e-15f * (1.0001f * F::magnitude(M, (3.0f * M * M + 2.0f * W) * 1.0001f,
+                                                           (W + fabsf(alpha)) * 1.0001f)) + 1e-30f;
+    const double v = f(p, (double)alpha);
+    if (v > bound) return 1;
+    if (v < -(double)bound) return -1;
+    return 0;
+}
+
+// Both FP64 filters: 0 when they cannot decide.
+template <class F, int N>
+__device__ __forceinline__ int filter_of(const F f, const Ball (&b)[N], float alpha, Tally &t) {
     t.evals++;
-    const int s = ev_sign(f(p, ev(alpha)));
+    const int s = plain_sign(f, b, alpha);
+    return s ? s : running_sign(f, b, alpha);
+}
+
+// The cascade: FP64 filter, integers when it cannot decide.
+template <class F, int N>
+__device__ __forceinline__ int sign_of(const F f, const Ball (&b)[N], float alpha, Tally &t) {
+    const int s = filter_of(f, b, alpha, t);
     if (s) return s;
     t.fallbacks++;
     return exact_sign(f, b, alpha, &t.range);
@@ -329,6 +401,15 @@ __device__ __forceinline__ bool tet_alpha(const Ball a1, const Ball a2, const Ba
     return sign_of(FTet{}, b, alpha, t) >= 0;
 }
 
+// The alpha decision where the FP64 filters can tell: 1 alpha, -1 not, else 0
+// (flat tetrahedra among them).
+__device__ __forceinline__ int tet_filter(const Ball a1, const Ball a2, const Ball a3,
+                                          const Ball a4, float alpha, Tally &t) {
+    const Ball b[4] = {a1, a2, a3, a4};
+    if (filter_of(FDet{}, b, alpha, t) == 0) return 0;
+    return filter_of(FTet{}, b, alpha, t);
+}
+
 __device__ __forceinline__ int orient_sign(const Ball a, const Ball b, const Ball c, const Ball d,
                                            Tally &t) {
     const Ball p[4] = {a, b, c, d};
@@ -339,6 +420,13 @@ __device__ __forceinline__ int insphere_sign(const Ball a, const Ball b, const B
                                              const Ball d, const Ball e, Tally &t) {
     const Ball p[5] = {a, b, c, d, e};
     return sign_of(FInsphere{}, p, 0.0f, t);
+}
+
+// insphere_sign where the FP64 filter can tell, else 0.
+__device__ __forceinline__ int insphere_filter(const Ball a, const Ball b, const Ball c,
+                                               const Ball d, const Ball e, Tally &t) {
+    const Ball p[5] = {a, b, c, d, e};
+    return filter_of(FInsphere{}, p, 0.0f, t);
 }
 
 __device__ __forceinline__ bool edge_attached(const Ball a1, const Ball a2, const Ball q,

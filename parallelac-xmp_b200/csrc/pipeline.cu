@@ -1687,7 +1687,7 @@ constexpr int kScanRefill = 16;  // idle lanes that trigger a refill
 // arithmetic; A.verify replays every certified decision too and counts
 // disagreements (C_CERT_BAD).  Survivors are recorded and mark their faces.
 template <int V>
-__global__ void __launch_bounds__(256, V == pac::kExact ? 2 : 4) k_tets_scan(TetArgs A, TetQueue Q, uint64_t nq,
+__global__ void __launch_bounds__(256, V == pac::kExact ? 3 : 4) k_tets_scan(TetArgs A, TetQueue Q, uint64_t nq,
                                                       unsigned long long *claim) {
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1;
@@ -1733,12 +1733,24 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 2 : 4) k_tets_scan(Tet
                     const Ball a1 = pac::ld_ball(&A.at[p]), a2 = pac::ld_ball(&A.at[v2]),
                                a3 = pac::ld_ball(&A.at[v3]), a4 = pac::ld_ball(&A.at[v4]);
                     float4 sph;
-                    bool mark;
-                    if constexpr (V == pac::kExact)
-                        mark = dec_tet<V>(a1, a2, a3, a4, A.alpha, sph, tally);
-                    else
+                    bool mark = true, live = true;
+                    if constexpr (V == pac::kExact) {
+                        // an alpha test that FP64 cannot decide (a flat
+                        // tetrahedron, a tie) waits for k_sos_resolve, so
+                        // that no lane holds up its warp with integers
+                        if (en.y & kAlphaOpen) {
+                            const int t = pac::ex::tet_filter(a1, a2, a3, a4, A.alpha, tally);
+                            mark = t > 0;
+                            if (t == 0) {
+                                const unsigned long long k = atomicAdd(&A.ctr[C_PEND], 1ull);
+                                if (k < A.pend_cap) A.pend[k] = en;
+                            }
+                        }
+                        const float3 x = pac::ex::tet_centre(a1, a2, a3, a4);
+                        sph = make_float4(x.x, x.y, x.z, 0.f);
+                    } else {
                         mark = pac::tet_alpha_g(pac::tet_group(a1, a2, a3), a2, a3, a4, A.alpha, sph);
-                    bool live = true;
+                    }
                     if (en.y & kAlphaOpen) {
                         live = mark && !(en.y & kRefuted);
                         late_alpha += mark;
@@ -1799,10 +1811,19 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 2 : 4) k_tets_scan(Tet
                 if (dec < 0 || A.verify) {
                     const float pa[3] = {ax, ay, az}, pb[3] = {bx, by, bz}, pc[3] = {cx, cy, cz},
                                 pd[3] = {dx, dy, dz}, pe[3] = {bb.x, bb.y, bb.z};
-                    const float res =
-                        dec_insphere<V>(pa, pb, pc, pd, pe, wa, wb, wc, wd, we, tally);
+                    float res;
+                    if constexpr (V == pac::kExact) {
+                        // the FP64 filter alone: what it cannot tell, a zero
+                        // among it, waits for k_sos_resolve, so that no lane
+                        // holds up its warp with integers
+                        res = (float)pac::ex::insphere_filter(
+                            Ball{ax, ay, az, wa}, Ball{bx, by, bz, wb}, Ball{cx, cy, cz, wc},
+                            Ball{dx, dy, dz, wd}, Ball{bb.x, bb.y, bb.z, we}, tally);
+                    } else {
+                        res = dec_insphere<V>(pa, pb, pc, pd, pe, wa, wb, wc, wd, we, tally);
+                    }
                     const int rdec = (orientation < 0 ? (res < 0) : (res > 0)) ? 1 : 0;
-                    if (dec >= 0 && dec != rdec) bad++;
+                    if (dec >= 0 && dec != rdec && !(V == pac::kExact && res == 0)) bad++;
                     if (dec < 0) {
                         dec = rdec;
                         if (res == 0) zero = true;
@@ -1837,26 +1858,46 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 2 : 4) k_tets_scan(Tet
     }
 }
 
-// Tetrahedra whose window holds an insphere value of exactly 0: the test
-// again, with the reference's simulation of simplicity for those balls
-// (AlphaComplexLargeData.cu:645-652, 659-667).
+// The tetrahedra that the scan left pending (no certain violator, but a ball
+// whose insphere value is exactly 0 or, in the exact mode, beyond the FP64
+// filters, or an alpha test beyond them): the test again, with the exact arithmetic and the reference's
+// simulation of simplicity for the zeros (AlphaComplexLargeData.cu:645-652,
+// 659-667).  A warp per tetrahedron, its lanes over the balls of a window
+// cell, the cells in the reference's order: the few pending ones are a chain of
+// integer evaluations each, so what counts is that they run beside each other
+// and outside the scan's warps (25,000 lattice-snapped balls, 156 zeros: a thread
+// per tetrahedron 2.4 ms, now 0.1; exact mode, 5,395 zeros and some 50,000 open
+// alpha tests: 37 ms here and 37 ms in the scan's lanes, now 3.5 and 1.4).
 template <int V>
-__global__ void k_sos_resolve(TetArgs A, uint64_t npend) {
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(128) k_sos_resolve(TetArgs A, uint64_t npend) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (t >= npend) return;
     uint2 pk = A.pend[t];
-    uint64_t p = pk.x;
-    int a = pk.y & 0xff, b = (pk.y >> 8) & 0xff, c = (pk.y >> 16) & 0xff;
+    const uint64_t p = pk.x;
+    const int a = pk.y & 0xff, b = (pk.y >> 8) & 0xff, c = (pk.y >> 16) & 0xff;
     const uint64_t e0 = A.eoff[p];
     const int deg = (int)(A.eoff[p + 1] - e0);
     const int W = (deg + 63) >> 6;
     const uint32_t *N = A.ER + e0;
-    uint32_t v[4] = {(uint32_t)p, N[a], N[b], N[c]};
+    const uint32_t v[4] = {(uint32_t)p, N[a], N[b], N[c]};
     Ball B[4];
     for (int k = 0; k < 4; k++) B[k] = pac::ld_ball(&A.at[v[k]]);
     Tally tally;
     float4 sphere;
-    dec_tet<V>(B[0], B[1], B[2], B[3], A.alpha, sphere, tally);
+    const bool mark = dec_tet<V>(B[0], B[1], B[2], B[3], A.alpha, sphere, tally);
+    if (pk.y & kAlphaOpen) {  // its alpha test was left open too
+        const bool refuted = pk.y & kRefuted;
+        if (lane == 0 && mark) {
+            bump(A.ctr, C_ALPHA_Q, 1);
+            bump(A.ctr, C_KILLED, refuted);
+        }
+        if (!mark || refuted) {
+            flush_tally<V>(lane == 0 ? tally : Tally{}, A.ctr);
+            return;
+        }
+        pk.y &= 0xffffffu;
+    }
     const MolGrid G = A.grids[mol_of(A.mol, p)];
     float pts[5][3], ws[5];
     int idx[5];
@@ -1867,13 +1908,20 @@ __global__ void k_sos_resolve(TetArgs A, uint64_t npend) {
         ws[k] = wt<V>(B[k].r);
         idx[k] = (int)A.orig[v[k]] + 1;
     }
-    float orientation = dec_orient<V>(pts[0], pts[1], pts[2], pts[3], ws[0], ws[1], ws[2], ws[3],
-                                      tally);
+    const float orient = pac::orient3d(pts[0], pts[1], pts[2], pts[3]);
+    const pac::cert::Insphere ct = pac::cert::setup(
+        B[0].x, B[0].y, B[0].z, B[0].r * B[0].r, B[1].x, B[1].y, B[1].z, B[1].r * B[1].r, B[2].x,
+        B[2].y, B[2].z, B[2].r * B[2].r, B[3].x, B[3].y, B[3].z, B[3].r * B[3].r, orient, sphere.x,
+        sphere.y, sphere.z, G.wmax);
+    const float orientation =
+        dec_orient<V>(pts[0], pts[1], pts[2], pts[3], ws[0], ws[1], ws[2], ws[3], tally);
+    if (lane) tally = Tally{};  // every lane took the same decisions so far
     int gridX = pac::cell_coord(sphere.x, G.minx, G.step);
     int gridY = pac::cell_coord(sphere.y, G.miny, G.step);
     int gridZ = pac::cell_coord(sphere.z, G.minz, G.step);
     int cc = lin3(gridX, gridY, gridZ, G.gx, G.gy);
     bool viol = false;
+    uint32_t calls = 0;
     for (int q = 0; q < 27 && !viol; q++) {
         uint32_t beg, end;
         if (q == 0) {
@@ -1891,26 +1939,40 @@ __global__ void k_sos_resolve(TetArgs A, uint64_t npend) {
             beg = A.cellbeg[gc];
             end = A.cellbeg[gc + 1];
         }
-        for (uint32_t e = beg; e < end && !viol; e++) {
-            if (e == v[0] || e == v[1] || e == v[2] || e == v[3]) continue;
-            const Ball atom = pac::ld_ball(&A.at[e]);
-            pts[4][0] = atom.x;
-            pts[4][1] = atom.y;
-            pts[4][2] = atom.z;
-            ws[4] = wt<V>(atom.r);
-            float result = dec_insphere<V>(pts[0], pts[1], pts[2], pts[3], pts[4], ws[0], ws[1],
-                                           ws[2], ws[3], ws[4], tally);
-            if (result == 0) {
-                idx[4] = (int)A.orig[e] + 1;
-                int status = 0;
-                result = (float)pac::sos_orientation(pts, ws, idx, &status, V == pac::kExact);
-                atomicAdd(&A.ctr[C_SOS], 1ull);
-                if (status == 1) atomicAdd(&A.ctr[C_SOS_RANGE], 1ull);
+        for (uint32_t base = beg; base < end && !viol; base += 32) {
+            const uint32_t e = base + lane;
+            bool hit = false, zero = false;
+            if (e < end && e != v[0] && e != v[1] && e != v[2] && e != v[3]) {
+                const Ball atom = pac::ld_ball(&A.at[e]);
+                const int dec = pac::cert::test(ct, atom.x, atom.y, atom.z, atom.r * atom.r);
+                hit = dec == 1;
+                if (dec < 0) {
+                    pts[4][0] = atom.x;
+                    pts[4][1] = atom.y;
+                    pts[4][2] = atom.z;
+                    ws[4] = wt<V>(atom.r);
+                    float result = dec_insphere<V>(pts[0], pts[1], pts[2], pts[3], pts[4], ws[0], ws[1],
+                                                   ws[2], ws[3], ws[4], tally);
+                    zero = result == 0;
+                    if (zero) {
+                        idx[4] = (int)A.orig[e] + 1;
+                        int status = 0;
+                        result = (float)pac::sos_orientation(pts, ws, idx, &status, V == pac::kExact);
+                        if (status == 1) atomicAdd(&A.ctr[C_SOS_RANGE], 1ull);
+                    }
+                    hit = orientation < 0 ? (result < 0) : (result > 0);
+                }
             }
-            viol = orientation < 0 ? (result < 0) : (result > 0);
+            // the zeros up to the first violator: those the reference's loop
+            // evaluates
+            const unsigned hits = __ballot_sync(kFull, hit), zeros = __ballot_sync(kFull, zero);
+            calls += __popc(hits ? zeros & (hits ^ (hits - 1)) : zeros);
+            viol = hits != 0;
         }
     }
-    flush_tally_thread<V>(tally, A.ctr);
+    flush_tally<V>(tally, A.ctr);
+    if (lane) return;
+    bump(A.ctr, C_SOS, calls);
     if (viol) return;
     unsigned long long q = atomicAdd(&A.ctr[C_SURV], 1ull);
     if (q < A.surv_cap) A.surv[q] = pk;
@@ -2757,7 +2819,7 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         }
         if (sp[1]) {
             CK(cudaEventRecord(ctx.ev[14], s));
-            k_sos_resolve<V><<<blocks_for(sp[1], 64), 64, 0, s>>>(T, sp[1]);
+            k_sos_resolve<V><<<blocks_for(sp[1], 4), 128, 0, s>>>(T, sp[1]);
             LAUNCH_CHECK(ctx);
             CK(cudaEventRecord(ctx.ev[15], s));
             ortho_pending = true;

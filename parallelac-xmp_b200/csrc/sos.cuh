@@ -12,74 +12,85 @@
 //
 // Here every input float is written as an integer multiple of a common
 // power of two and the minors are evaluated with two's-complement integers
-// of kLimbs 32-bit limbs.  This runs only in the fallback kernel that
-// resolves the rare exact zeros, so it favours simplicity over speed.
+// of 32-bit limbs: as few as the inputs' range needs, at most kLimbs.  A
+// product costs limbs squared and the integers live in local memory, so the
+// 8 limbs that molecules need (coordinates below 128 with bits down to 2^-50)
+// take a sixth of kLimbs' time.
 #pragma once
 #include <cstdint>
 
 namespace pac {
 
-constexpr int kLimbs = 20;  // 640-bit integers
+constexpr int kLimbs = 20;      // 640-bit integers: the widest
+constexpr int kLimbsShort = 8;  // 256-bit
 
+template <int L>
 struct BigInt {
-    uint32_t w[kLimbs];
+    uint32_t w[L];
 };
 
-static __device__ inline void bi_zero(BigInt &r) {
+template <int L>
+static __device__ inline void bi_zero(BigInt<L> &r) {
 #pragma unroll
-    for (int i = 0; i < kLimbs; i++) r.w[i] = 0;
+    for (int i = 0; i < L; i++) r.w[i] = 0;
 }
-static __device__ inline void bi_add(BigInt &r, const BigInt &a, const BigInt &b) {
+template <int L>
+static __device__ inline void bi_add(BigInt<L> &r, const BigInt<L> &a, const BigInt<L> &b) {
     uint64_t c = 0;
-    for (int i = 0; i < kLimbs; i++) {
+    for (int i = 0; i < L; i++) {
         uint64_t t = (uint64_t)a.w[i] + b.w[i] + c;
         r.w[i] = (uint32_t)t;
         c = t >> 32;
     }
 }
-static __device__ inline void bi_negate(BigInt &r) {
+template <int L>
+static __device__ inline void bi_negate(BigInt<L> &r) {
     uint64_t c = 1;
-    for (int i = 0; i < kLimbs; i++) {
+    for (int i = 0; i < L; i++) {
         uint64_t t = (uint64_t)(~r.w[i]) + c;
         r.w[i] = (uint32_t)t;
         c = t >> 32;
     }
 }
-static __device__ inline void bi_sub(BigInt &r, const BigInt &a, const BigInt &b) {
-    BigInt nb = b;
+template <int L>
+static __device__ inline void bi_sub(BigInt<L> &r, const BigInt<L> &a, const BigInt<L> &b) {
+    BigInt<L> nb = b;
     bi_negate(nb);
     bi_add(r, a, nb);
 }
-static __device__ inline int bi_sign(const BigInt &a) {
-    if (a.w[kLimbs - 1] & 0x80000000u) return -1;
-    for (int i = 0; i < kLimbs; i++)
+template <int L>
+static __device__ inline int bi_sign(const BigInt<L> &a) {
+    if (a.w[L - 1] & 0x80000000u) return -1;
+    for (int i = 0; i < L; i++)
         if (a.w[i]) return 1;
     return 0;
 }
-static __device__ inline void bi_mul(BigInt &r, const BigInt &a, const BigInt &b) {
-    BigInt x = a, y = b;
+template <int L>
+static __device__ inline void bi_mul(BigInt<L> &r, const BigInt<L> &a, const BigInt<L> &b) {
+    BigInt<L> x = a, y = b;
     bool neg = false;
     if (bi_sign(x) < 0) { bi_negate(x); neg = !neg; }
     if (bi_sign(y) < 0) { bi_negate(y); neg = !neg; }
-    uint32_t acc[kLimbs];
-    for (int i = 0; i < kLimbs; i++) acc[i] = 0;
-    for (int i = 0; i < kLimbs; i++) {
+    uint32_t acc[L];
+    for (int i = 0; i < L; i++) acc[i] = 0;
+    for (int i = 0; i < L; i++) {
         uint32_t xi = x.w[i];
         if (!xi) continue;
         uint32_t carry = 0;
-        for (int j = 0; i + j < kLimbs; j++) {
+        for (int j = 0; i + j < L; j++) {
             // acc[i+j] + xi*y[j] + carry, with 64-bit intermediate
             uint64_t t = (uint64_t)xi * y.w[j] + acc[i + j] + carry;
             acc[i + j] = (uint32_t)t;
             carry = (uint32_t)(t >> 32);
         }
     }
-    for (int i = 0; i < kLimbs; i++) r.w[i] = acc[i];
+    for (int i = 0; i < L; i++) r.w[i] = acc[i];
     if (neg) bi_negate(r);
 }
 
 // float -> integer at scale 2^scale (the float must be a multiple of it)
-static __device__ inline void bi_from_float(BigInt &r, float f, int scale) {
+template <int L>
+static __device__ inline void bi_from_float(BigInt<L> &r, float f, int scale) {
     bi_zero(r);
     uint32_t u = __float_as_uint(f);
     uint32_t ex = (u >> 23) & 0xffu, fr = u & 0x7fffffu;
@@ -88,10 +99,10 @@ static __device__ inline void bi_from_float(BigInt &r, float f, int scale) {
     if (!m) return;
     int sh = e - scale;
     int limb = sh >> 5, bit = sh & 31;
-    if (limb < kLimbs) {
+    if (limb < L) {
         uint64_t v = (uint64_t)m << bit;
         r.w[limb] = (uint32_t)v;
-        if (limb + 1 < kLimbs) r.w[limb + 1] = (uint32_t)(v >> 32);
+        if (limb + 1 < L) r.w[limb + 1] = (uint32_t)(v >> 32);
     }
     if (u >> 31) bi_negate(r);
 }
@@ -140,23 +151,25 @@ constexpr uint64_t kSosFlip = (1ull << 1) | (1ull << 3) | (1ull << 7) | (1ull <<
                               (1ull << 37) | (1ull << 39) | (1ull << 41) | (1ull << 44) |
                               (1ull << 46);
 
+template <int N>
 struct SosPoints {
-    BigInt c[5][3];  // coordinates at scale 2^E
-    BigInt lift[5];  // |p|^2 - w at scale 2^(2E)
-    BigInt w[5];     // w at scale 2^(2E)
+    BigInt<N> c[5][3];  // coordinates at scale 2^E
+    BigInt<N> lift[5];  // |p|^2 - w at scale 2^(2E)
+    BigInt<N> w[5];     // w at scale 2^(2E)
 };
 
 // 4x4 orientation with rows (X, Y, L, 1), expanded as in
 // orient3dexact_l_w (predicates.h:4466-4506).
-static __device__ __noinline__ int sos_det3(const BigInt *X, const BigInt *Y, const BigInt *L) {
-    BigInt m[6], t1, t2;
+template <int N>
+static __device__ __noinline__ int sos_det3(const BigInt<N> *X, const BigInt<N> *Y, const BigInt<N> *L) {
+    BigInt<N> m[6], t1, t2;
     const int P[6] = {0, 1, 2, 3, 0, 1}, Q[6] = {1, 2, 3, 0, 2, 3};  // ab bc cd da ac bd
     for (int k = 0; k < 6; k++) {
         bi_mul(t1, L[Q[k]], Y[P[k]]);
         bi_mul(t2, L[P[k]], Y[Q[k]]);
         bi_sub(m[k], t1, t2);
     }
-    BigInt cda, dab, abc, bcd, acc;
+    BigInt<N> cda, dab, abc, bcd, acc;
     bi_add(cda, m[2], m[3]);
     bi_add(cda, cda, m[4]);
     bi_add(dab, m[3], m[0]);
@@ -176,8 +189,9 @@ static __device__ __noinline__ int sos_det3(const BigInt *X, const BigInt *Y, co
 }
 
 // 3x3 orientation with rows (X, L, 1) (orient2dexact_l_w, predicates.h:4575-4596).
-static __device__ __noinline__ int sos_det2(const BigInt *X, const BigInt *L) {
-    BigInt d, t, acc;
+template <int N>
+static __device__ __noinline__ int sos_det2(const BigInt<N> *X, const BigInt<N> *L) {
+    BigInt<N> d, t, acc;
     bi_sub(d, L[1], L[2]);
     bi_mul(acc, X[0], d);
     bi_sub(d, L[2], L[0]);
@@ -189,9 +203,10 @@ static __device__ __noinline__ int sos_det2(const BigInt *X, const BigInt *L) {
     return bi_sign(acc);
 }
 
-static __device__ __noinline__ int sos_minor(const SosPoints &s, int depth) {
+template <int N>
+static __device__ __noinline__ int sos_minor(const SosPoints<N> &s, int depth) {
     const SosStep st = kSosSteps[depth];
-    BigInt X[4], Y[4], L[4];
+    BigInt<N> X[4], Y[4], L[4];
     if (st.kind == 3) {
         for (int r = 0; r < 4; r++) {
             int p = st.rows[r];
@@ -210,20 +225,51 @@ static __device__ __noinline__ int sos_minor(const SosPoints &s, int depth) {
         return sos_det2(X, L);
     }
     int a = st.rows[0], b = st.rows[1];
-    BigInt t;
+    BigInt<N> t;
     if (!st.lifted) {
         bi_sub(t, s.c[a][st.perm[0]], s.c[b][st.perm[0]]);
         return bi_sign(t);
     }
     // orient1dexact_l_w with the lifted coordinate (predicates.h:4605-4647):
     // (|a|^2 - |b|^2) + (w_a - w_b) = (lift_a + 2 w_a) - (lift_b + 2 w_b)
-    BigInt la, lb;
+    BigInt<N> la, lb;
     bi_add(la, s.lift[a], s.w[a]);
     bi_add(la, la, s.w[a]);
     bi_add(lb, s.lift[b], s.w[b]);
     bi_add(lb, lb, s.w[b]);
     bi_sub(t, la, lb);
     return bi_sign(t);
+}
+
+// The minors of the points p[ord[0..4]] in order until one is nonzero: its sign
+// and depth, or 0 with depth 49.
+template <int N>
+static __device__ __noinline__ int sos_sequence(const float (*p)[3], const float *w, const int *ord,
+                                                int emin, bool radii, int &depth) {
+    SosPoints<N> s;
+    for (int i = 0; i < 5; i++) {
+        BigInt<N> sq, acc;
+        bi_zero(acc);
+        for (int k = 0; k < 3; k++) {
+            bi_from_float(s.c[i][k], p[ord[i]][k], emin);
+            bi_mul(sq, s.c[i][k], s.c[i][k]);
+            bi_add(acc, acc, sq);
+        }
+        if (radii) {
+            BigInt<N> r;
+            bi_from_float(r, w[ord[i]], emin);
+            bi_mul(s.w[i], r, r);
+        } else {
+            bi_from_float(s.w[i], w[ord[i]], 2 * emin);
+        }
+        bi_sub(s.lift[i], acc, s.w[i]);
+    }
+    int sign = 0;
+    for (depth = 1; depth <= 48; depth++) {
+        sign = sos_minor(s, depth);
+        if (sign) break;
+    }
+    return sign;
 }
 
 // Sign of orientation4SoS_w(p[0..4], w[0..4], idx[0..4]).  Returns +1/-1;
@@ -256,29 +302,10 @@ static __device__ __noinline__ int sos_orientation(const float (*p)[3], const fl
             emax = max(emax, e + 24);
         }
     *status = ((emax - emin) * 4 + 12 > kLimbs * 32 - 2) ? 1 : 0;
-    SosPoints s;
-    for (int i = 0; i < 5; i++) {
-        BigInt sq, acc;
-        bi_zero(acc);
-        for (int k = 0; k < 3; k++) {
-            bi_from_float(s.c[i][k], p[ord[i]][k], emin);
-            bi_mul(sq, s.c[i][k], s.c[i][k]);
-            bi_add(acc, acc, sq);
-        }
-        if (radii) {
-            BigInt r;
-            bi_from_float(r, w[ord[i]], emin);
-            bi_mul(s.w[i], r, r);
-        } else {
-            bi_from_float(s.w[i], w[ord[i]], 2 * emin);
-        }
-        bi_sub(s.lift[i], acc, s.w[i]);
-    }
-    int sign = 0, depth = 0;
-    for (depth = 1; depth <= 48; depth++) {
-        sign = sos_minor(s, depth);
-        if (sign) break;
-    }
+    int depth = 0;
+    int sign = (emax - emin) * 4 + 12 <= kLimbsShort * 32 - 2
+                   ? sos_sequence<kLimbsShort>(p, w, ord, emin, radii, depth)
+                   : sos_sequence<kLimbs>(p, w, ord, emin, radii, depth);
     if (!sign) {
         sign = 1;
         depth = 49;
