@@ -321,82 +321,127 @@ __device__ __forceinline__ void flush_tally_thread(const Tally &t, unsigned long
 }
 
 // ------------------------------------------------------------------ scan
-// Exclusive prefix sum of n values into out[0..n], out[n] = total.
-template <class Tin>
-__global__ void k_scan_reduce(const Tin *in, uint64_t n, uint64_t *bsum) {
-    __shared__ uint64_t s[32];
-    uint64_t base = (uint64_t)blockIdx.x * 4096;
-    uint64_t acc = 0;
-    for (int k = 0; k < 4; k++) {
-        uint64_t i = base + (uint64_t)k * 1024 + threadIdx.x;
-        if (i < n) acc += (uint64_t)in[i];
-    }
-    acc = warp_sum(acc);
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = acc;
+// Exclusive prefix sum of n values into out[0..n], out[n] = total.  A block
+// of 8 warps takes kScanTile values, a warp 512 consecutive ones held in
+// registers (16 coalesced loads), scanned by shuffles.  What bounds it at the
+// sizes of one molecule is launches and barriers: one tile is one launch, up to
+// kScanWide tiles are two (each block adds up the sums of the tiles before
+// it), more are three.  Against three launches with shared-memory scans of 20
+// barriers per 1,024 values: 13 -> 5 us of kernel time a scan at 211 balls, 16 ->
+// 13 us at 25,000 (of that about 2.5 us per launch).
+constexpr int kScanTile = 4096;
+constexpr uint64_t kScanWide = 1024;
+
+// sum of the block's values v (all threads get it)
+__device__ __forceinline__ unsigned long long block_sum(unsigned long long v) {
+    __shared__ unsigned long long s[8];
+    v = warp_sum(v);
     __syncthreads();
-    if (threadIdx.x < 32) {
-        uint64_t v = s[threadIdx.x];
-        v = warp_sum(v);
-        if (threadIdx.x == 0) bsum[blockIdx.x] = v;
-    }
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) v += s[w];
+    return v;
 }
-__global__ void k_scan_blocks(uint64_t *bsum, uint64_t nb) {
-    // single block: exclusive scan of nb block sums in place
-    __shared__ uint64_t s[1024];
-    uint64_t carry = 0;
-    for (uint64_t base = 0; base < nb; base += 1024) {
-        uint64_t i = base + threadIdx.x;
-        uint64_t v = i < nb ? bsum[i] : 0;
-        s[threadIdx.x] = v;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {
-            uint64_t t = threadIdx.x >= (unsigned)o ? s[threadIdx.x - o] : 0;
-            __syncthreads();
-            s[threadIdx.x] += t;
-            __syncthreads();
+template <class Tin>
+__global__ void __launch_bounds__(256) k_scan_reduce(const Tin *in, uint64_t n, uint64_t *bsum) {
+    const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
+    unsigned long long acc = 0;
+#pragma unroll
+    for (int k = 0; k < kScanTile / 256; k++) {
+        const uint64_t i = base + (uint64_t)k * 256 + threadIdx.x;
+        if (i < n) acc += (unsigned long long)in[i];
+    }
+    acc = block_sum(acc);
+    if (threadIdx.x == 0) bsum[blockIdx.x] = acc;
+}
+// exclusive prefix sums of the nb tile sums, in place, in one block
+__global__ void __launch_bounds__(256) k_scan_blocks(uint64_t *bsum, uint64_t nb) {
+    __shared__ unsigned long long s[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long carry = 0;
+    for (uint64_t base = 0; base < nb; base += 256) {
+        const uint64_t i = base + threadIdx.x;
+        const unsigned long long v = i < nb ? bsum[i] : 0;
+        unsigned long long incl = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long t = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += t;
         }
-        if (i < nb) bsum[i] = carry + s[threadIdx.x] - v;
-        uint64_t tot = s[1023];
         __syncthreads();
+        if (lane == 31) s[warp] = incl;
+        __syncthreads();
+        unsigned long long before = carry, tot = 0;
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            if (w < warp) before += s[w];
+            tot += s[w];
+        }
+        if (i < nb) bsum[i] = before + incl - v;
         carry += tot;
     }
-    if (threadIdx.x == 0) bsum[nb] = carry;
 }
+// bsum: the tiles' sums (summed = false) or their prefix sums (true); unused
+// when there is one tile
 template <class Tin, class Tout>
-__global__ void k_scan_apply(const Tin *in, uint64_t n, const uint64_t *bsum, Tout *out) {
-    __shared__ uint64_t s[1024];
-    uint64_t base = (uint64_t)blockIdx.x * 4096;
-    uint64_t carry = bsum[blockIdx.x];
-    for (int k = 0; k < 4; k++) {
-        uint64_t i = base + (uint64_t)k * 1024 + threadIdx.x;
-        uint64_t v = i < n ? (uint64_t)in[i] : 0;
-        s[threadIdx.x] = v;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {
-            uint64_t t = threadIdx.x >= (unsigned)o ? s[threadIdx.x - o] : 0;
-            __syncthreads();
-            s[threadIdx.x] += t;
-            __syncthreads();
-        }
-        if (i < n) out[i] = (Tout)(carry + s[threadIdx.x] - v);
-        uint64_t tot = s[1023];
-        __syncthreads();
-        carry += tot;
+__global__ void __launch_bounds__(256) k_scan_apply(const Tin *in, uint64_t n, const uint64_t *bsum,
+                                                    bool summed, Tout *out) {
+    __shared__ unsigned long long s[8];
+    constexpr int kPer = kScanTile / 256;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)warp * (32 * kPer);
+    unsigned long long carry = 0;
+    if (summed) {
+        carry = bsum[blockIdx.x];
+    } else {
+        for (uint64_t b = threadIdx.x; b < blockIdx.x; b += 256) carry += bsum[b];
+        if (blockIdx.x) carry = block_sum(carry);
     }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = (Tout)bsum[gridDim.x];
+    Tin v[kPer];
+    unsigned long long mine = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        const uint64_t i = base + (uint64_t)k * 32 + lane;
+        v[k] = i < n ? in[i] : Tin(0);
+        mine += (unsigned long long)v[k];
+    }
+    mine = warp_sum(mine);
+    if (lane == 0) s[warp] = mine;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; w++)
+        if (w < warp) carry += s[w];
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        const uint64_t i = base + (uint64_t)k * 32 + lane;
+        unsigned long long incl = (unsigned long long)v[k];
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long t = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (i < n) out[i] = (Tout)(carry + incl - (unsigned long long)v[k]);
+        if (i + 1 == n) out[n] = (Tout)(carry + incl);
+        carry += __shfl_sync(kFull, incl, 31);
+    }
+    if (n == 0 && threadIdx.x == 0) out[0] = 0;
 }
 
 template <class Tin, class Tout>
 static int exclusive_scan(pac::Ctx &ctx, const Tin *in, uint64_t n, Tout *out) {
-    uint64_t nb = (n + 4095) / 4096;
-    if (nb == 0) nb = 1;
-    uint64_t *bsum = ctx.arena.alloc_n<uint64_t>(nb + 1);
-    if (!bsum) return PAC_ERR_OOM;
-    k_scan_reduce<Tin><<<(unsigned)nb, 1024, 0, ctx.stream>>>(in, n, bsum);
-    LAUNCH_CHECK(ctx);
-    k_scan_blocks<<<1, 1024, 0, ctx.stream>>>(bsum, nb);
-    LAUNCH_CHECK(ctx);
-    k_scan_apply<Tin, Tout><<<(unsigned)nb, 1024, 0, ctx.stream>>>(in, n, bsum, out);
+    const uint64_t nb = std::max<uint64_t>(1, (n + kScanTile - 1) / kScanTile);
+    uint64_t *bsum = nullptr;
+    if (nb > 1) {
+        bsum = ctx.arena.alloc_n<uint64_t>(nb);
+        if (!bsum) return PAC_ERR_OOM;
+        k_scan_reduce<Tin><<<(unsigned)nb, 256, 0, ctx.stream>>>(in, n, bsum);
+        LAUNCH_CHECK(ctx);
+    }
+    if (nb > kScanWide) {
+        k_scan_blocks<<<1, 256, 0, ctx.stream>>>(bsum, nb);
+        LAUNCH_CHECK(ctx);
+    }
+    k_scan_apply<Tin, Tout><<<(unsigned)nb, 256, 0, ctx.stream>>>(in, n, bsum, nb > kScanWide, out);
     LAUNCH_CHECK(ctx);
     return PAC_OK;
 }
@@ -617,15 +662,21 @@ __global__ void __launch_bounds__(256) k_edges(uint64_t n, const float4 *__restr
     }
 }
 
-// words of link matrix per ball
-__global__ void k_link_size(uint64_t n, const uint64_t *eoff, uint64_t *lsize,
-                            unsigned long long *ctr) {
-    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    uint64_t deg = eoff[p + 1] - eoff[p];
-    uint64_t W = (deg + 63) >> 6;
-    lsize[p] = deg * W;
-    atomicMax(&ctr[C_MAXDEG], (unsigned long long)deg);
+// words of link matrix per ball; the largest degree through one atomic per
+// block (one per ball serialised on its address: 18 us at 25,000 balls)
+__global__ void __launch_bounds__(256) k_link_size(uint64_t n, const uint64_t *eoff, uint64_t *lsize,
+                                                   unsigned long long *ctr) {
+    __shared__ unsigned m[8];
+    const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t deg = p < n ? eoff[p + 1] - eoff[p] : 0;
+    if (p < n) lsize[p] = deg * ((deg + 63) >> 6);
+    const unsigned w = __reduce_max_sync(kFull, (unsigned)min(deg, (uint64_t)0xffffffffu));
+    if ((threadIdx.x & 31) == 0) m[threadIdx.x >> 5] = w;
+    __syncthreads();
+    if (threadIdx.x) return;
+    unsigned top = 0;
+    for (int k = 0; k < 8; k++) top = max(top, m[k]);
+    if (top > *(volatile unsigned long long *)&ctr[C_MAXDEG]) atomicMax(&ctr[C_MAXDEG], (unsigned long long)top);
 }
 
 // ------------------------------------------------------------------ triangles
@@ -1988,43 +2039,36 @@ __global__ void __launch_bounds__(128) k_sos_resolve(TetArgs A, uint64_t npend) 
     mark_face(A.faces, A.loff[v2], (deg2 + 63) >> 6, mb, mc);
 }
 
-// Survivors to per-ball rows: scatter, then order each ball's rows by
-// (a, b, c) -- the order in which the reference enumerates them.
+// Survivors to per-ball rows, ordered by (a, b, c) -- the order in which the
+// reference enumerates them: k_tet_scatter collects each ball's keys, then a
+// thread per tetrahedron counts the smaller keys of its ball (a few to a few
+// tens, in L1) and writes its row there.  (A thread per ball sorting by
+// insertion: 29 us at 211 balls, 56 at 25,000.)
+__device__ __forceinline__ uint32_t key_order(uint32_t k) {
+    return ((k & 0xff) << 16) | (k & 0xff00) | ((k >> 16) & 0xff);
+}
 __global__ void k_tet_scatter(const uint2 *surv, uint64_t ns, const uint64_t *toff,
                               uint32_t *cursor, uint32_t *keys, uint64_t p_lo, uint64_t p_hi) {
     uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ns) return;
     uint2 s = surv[t];
     if (s.x < p_lo || s.x >= p_hi) return;  // a slab's halo: not this pass's output
-    keys[toff[s.x] + atomicAdd(&cursor[s.x], 1u)] = s.y;
+    keys[toff[s.x] + atomicAdd(&cursor[s.x], 1u)] = key_order(s.y);
 }
-__global__ void k_tet_sort_emit(uint64_t n, const uint64_t *toff, uint32_t *keys,
-                                const uint64_t *eoff, const uint32_t *ER, const uint32_t *orig,
-                                uint32_t *out) {
-    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    uint64_t b = toff[p], e = toff[p + 1];
-    for (uint64_t i = b + 1; i < e; i++) {
-        uint32_t v = keys[i];
-        uint32_t vk = ((v & 0xff) << 16) | (v & 0xff00) | ((v >> 16) & 0xff);
-        uint64_t j = i;
-        while (j > b) {
-            uint32_t u = keys[j - 1];
-            uint32_t uk = ((u & 0xff) << 16) | (u & 0xff00) | ((u >> 16) & 0xff);
-            if (uk <= vk) break;
-            keys[j] = u;
-            j--;
-        }
-        keys[j] = v;
-    }
-    const uint32_t *N = ER + eoff[p];
-    const uint32_t o1 = orig[p];
-    for (uint64_t i = b; i < e; i++) {
-        uint32_t k = keys[i];
-        uint4 t = make_uint4(o1, orig[N[k & 0xff]], orig[N[(k >> 8) & 0xff]],
-                             orig[N[(k >> 16) & 0xff]]);
-        *(uint4 *)&out[4 * i] = t;
-    }
+__global__ void k_tet_emit(const uint2 *surv, uint64_t ns, const uint64_t *toff, const uint32_t *keys,
+                           const uint64_t *eoff, const uint32_t *ER, const uint32_t *orig,
+                           uint32_t *out, uint64_t p_lo, uint64_t p_hi) {
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ns) return;
+    const uint2 s = surv[t];
+    if (s.x < p_lo || s.x >= p_hi) return;
+    const uint64_t b = toff[s.x], e = toff[s.x + 1];
+    const uint32_t mine = key_order(s.y);
+    uint64_t at = b;
+    for (uint64_t i = b; i < e; i++) at += __ldg(&keys[i]) < mine;
+    const uint32_t *N = ER + eoff[s.x];
+    *(uint4 *)&out[4 * at] = make_uint4(orig[s.x], orig[N[s.y & 0xff]], orig[N[(s.y >> 8) & 0xff]],
+                                        orig[N[(s.y >> 16) & 0xff]]);
 }
 __global__ void k_map4(uint64_t nq, const uint32_t *orig, uint32_t *tets) {
     uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2302,18 +2346,20 @@ __global__ void __launch_bounds__(256) k_edge_final(uint64_t p_lo, uint64_t n,
 }
 
 // ------------------------------------------------------------------ emission
-__global__ void k_emit_edges(uint64_t n, const uint64_t *eoff, const uint32_t *ER,
-                             const uint8_t *eflag, const uint64_t *epos, const uint32_t *orig,
-                             uint32_t *out) {
-    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    uint32_t o = orig[p];
-    for (uint64_t k = eoff[p]; k < eoff[p + 1]; k++)
-        if (eflag[k]) {
-            uint64_t q = epos[k];
-            out[2 * q] = o;
-            out[2 * q + 1] = orig[ER[k]];
-        }
+// a warp per ball, its lanes over the ball's alpha edges (a thread per ball
+// walking its row alone: 40 us at 211 balls, 112 at 25,000)
+__global__ void __launch_bounds__(256) k_emit_edges(uint64_t n, const uint64_t *eoff, const uint32_t *ER,
+                                                    const uint8_t *eflag, const uint64_t *epos,
+                                                    const uint32_t *orig, uint32_t *out) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t p = warp; p < n; p += nwarps) {
+        const uint32_t o = orig[p];
+        const uint64_t end = eoff[p + 1];
+        for (uint64_t k = eoff[p] + lane; k < end; k += 32)
+            if (eflag[k]) *(uint2 *)&out[2 * epos[k]] = make_uint2(o, orig[ER[k]]);
+    }
 }
 __global__ void __launch_bounds__(256) k_emit_tris(uint64_t p_lo, uint64_t n, const uint64_t *eoff,
                                                    const uint32_t *ER, const uint64_t *loff,
@@ -2646,7 +2692,6 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
     T.maxlen = ctr + C_MAXLEN;
     T.refute = cfg.refute ? 1 : 0;
     T.verify = cfg.verify ? 1 : 0;
-    T.scan_claim = std::max(32, cfg.scan_claim);
     T.tcount = ar.alloc_n<uint32_t>(n);
     uint64_t *toff = ar.alloc_n<uint64_t>(n + 1);
     if (!T.tcount || !toff) return PAC_ERR_OOM;
@@ -2773,7 +2818,12 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
             CK(cudaMemsetAsync(claim, 0, sizeof(unsigned long long), s));
             if (queued) {
                 CK(cudaEventRecord(ctx.ev[14], s));
-                k_tets_scan<V><<<148 * std::max(1, cfg.scan_blocks), 256, 0, s>>>(T, Q, queued, claim);
+                // claims no larger than an equal share: a short queue occupies
+                // every warp
+                const unsigned grid = 148u * (unsigned)std::max(1, cfg.scan_blocks);
+                T.scan_claim = (int)std::min<uint64_t>(std::max(32, cfg.scan_claim),
+                                                       std::max<uint64_t>(32, queued / (8ull * grid)));
+                k_tets_scan<V><<<grid, 256, 0, s>>>(T, Q, queued, claim);
                 LAUNCH_CHECK(ctx);
                 CK(cudaEventRecord(ctx.ev[15], s));
                 ortho_pending = true;
@@ -2858,8 +2908,8 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         k_tet_scatter<<<blocks_for(ns, 256), 256, 0, s>>>(T.surv, ns, toff, cursor, keys, own_lo,
                                                           own_hi);
         LAUNCH_CHECK(ctx);
-        k_tet_sort_emit<<<blocks_for(n, 128), 128, 0, s>>>(n, toff, keys, eoff, ER, orig,
-                                                           out.d_tets);
+        k_tet_emit<<<blocks_for(ns, 256), 256, 0, s>>>(T.surv, ns, toff, keys, eoff, ER, orig,
+                                                       out.d_tets, own_lo, own_hi);
         LAUNCH_CHECK(ctx);
     }
     if (in.to_host && (rc = pac::list_to_host_async(ctx, 2, out.d_tets, 4 * nQ, &out.h_tets)))
@@ -2917,7 +2967,7 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
     CK(cudaStreamSynchronize(s));
     out.d_edges = ar.alloc_n<uint32_t>(2 * nEf);
     if (!out.d_edges) return PAC_ERR_OOM;
-    k_emit_edges<<<blocks_for(n, 256), 256, 0, s>>>(n, eoff, ER, eflag, epos, orig, out.d_edges);
+    k_emit_edges<<<warp_blocks(n), 256, 0, s>>>(n, eoff, ER, eflag, epos, orig, out.d_edges);
     LAUNCH_CHECK(ctx);
     if (in.to_host && (rc = pac::list_to_host_async(ctx, 0, out.d_edges, 2 * nEf, &out.h_edges)))
         return rc;
