@@ -174,13 +174,6 @@ struct EventSet {
     EventSet &operator=(const EventSet &) = delete;
 };
 
-__global__ void k_check_finite(const float4 *b, uint64_t n, int *bad) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4 v = b[i];
-    if (!isfinite(v.x) || !isfinite(v.y) || !isfinite(v.z) || !isfinite(v.w)) *bad = 1;
-}
-
 // Launch shapes for the autotuner (pac_options.autotune): blocks per SM of
 // the tetrahedron enumeration (balls of at most 64 upper neighbours; larger
 // ones) and of the orthosphere scan, and the queue entries a scan warp claims
@@ -199,16 +192,6 @@ int run(pac_ctx *ctx, const float4 *d_balls, uint64_t n, uint32_t n_mol,
     pac::Ctx &c = ctx->c;
     if (!std::isfinite(sol) || !std::isfinite(alpha))
         return pac::set_error(PAC_ERR_INVALID_ARG, "sol_rad and alpha must be finite");
-    int *bad = c.arena.alloc_n<int>(1);
-    if (!bad) return PAC_ERR_OOM;
-    cudaMemsetAsync(bad, 0, sizeof(int), c.stream);
-    k_check_finite<<<(unsigned)((n + 255) / 256), 256, 0, c.stream>>>(d_balls, n, bad);
-    int hbad = 0;
-    cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c.stream);
-    cudaError_t e = cudaStreamSynchronize(c.stream);
-    if (e != cudaSuccess)
-        return pac::set_error(PAC_ERR_CUDA, std::string("input check: ") + cudaGetErrorString(e));
-    if (hbad) return pac::set_error(PAC_ERR_INVALID_ARG, "non-finite ball coordinate or radius");
     // the alpha-tetrahedron queue: a quarter of the free memory at the
     // context's first pass, at most 12 GiB (8 B per entry); a pass whose
     // queued tetrahedra exceed it runs in chunks
@@ -266,7 +249,7 @@ int run(pac_ctx *ctx, const float4 *d_balls, uint64_t n, uint32_t n_mol,
         }
     }
     if (rc == PAC_OK) {
-        e = cudaStreamSynchronize(c.stream);
+        const cudaError_t e = cudaStreamSynchronize(c.stream);
         if (e != cudaSuccess)
             return pac::set_error(PAC_ERR_CUDA, std::string("pass: ") + cudaGetErrorString(e));
     }

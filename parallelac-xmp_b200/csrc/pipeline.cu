@@ -50,7 +50,7 @@ constexpr unsigned kFull = 0xffffffffu;
 // device-side counters (one slot each)
 enum Counter {
     C_CAND_E, C_ALPHA_E, C_CAND_T, C_ALPHA_T, C_CAND_Q, C_ALPHA_Q, C_INSPHERE, C_SOS,
-    C_OOB, C_SURV, C_PEND, C_MAXDEG, C_SOS_RANGE, C_BADDEG, C_NEXT, C_FILTER, C_FALLBACK,
+    C_OOB, C_SURV, C_PEND, C_MAXDEG, C_SOS_RANGE, C_NONFINITE, C_NEXT, C_FILTER, C_FALLBACK,
     C_KILLED, C_KTESTS, C_CERT, C_CERT_BAD,
     C_MAXLEN,                 // largest squared alpha-edge length (bits of a binary32)
     C_CLASS, C_TAKE = C_CLASS + 3,  // balls per enumeration class, and handed out of each
@@ -454,12 +454,15 @@ __global__ void k_mol_ids(const uint64_t *off, uint32_t n_mol, uint32_t *mol) {
 }
 
 // min/max of raw x, y, z, r per molecule (AlphaComplexLargeData.cu:1088-1110).
-// Floats are compared through an order-preserving int key.
-__global__ void k_bbox(const float4 *balls, uint64_t n, const uint32_t *mol, int *mm) {
+// Floats are compared through an order-preserving int key.  Non-finite
+// coordinates and radii are reported in ctr[C_NONFINITE].
+__global__ void k_bbox(const float4 *balls, uint64_t n, const uint32_t *mol, int *mm,
+                       unsigned long long *ctr) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool act = i < n;
     uint32_t m = act ? mol_of(mol, i) : 0xffffffffu;
     float4 b = act ? balls[i] : make_float4(0, 0, 0, 0);
+    if (!isfinite(b.x) || !isfinite(b.y) || !isfinite(b.z) || !isfinite(b.w)) ctr[C_NONFINITE] = 1;
     int k[4] = {fkey(b.x), fkey(b.y), fkey(b.z), fkey(b.w)};
     uint32_t m0 = __shfl_sync(kFull, m, 0);
     bool uniform = __all_sync(kFull, act && m == m0);
@@ -664,13 +667,13 @@ __global__ void __launch_bounds__(256) k_edges(uint64_t n, const float4 *__restr
 
 // words of link matrix per ball; the largest degree through one atomic per
 // block (one per ball serialised on its address: 18 us at 25,000 balls)
-__global__ void __launch_bounds__(256) k_link_size(uint64_t n, const uint64_t *eoff, uint64_t *lsize,
+__global__ void __launch_bounds__(256) k_link_size(uint64_t n, const uint32_t *ecount, uint64_t *lsize,
                                                    unsigned long long *ctr) {
     __shared__ unsigned m[8];
     const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t deg = p < n ? eoff[p + 1] - eoff[p] : 0;
+    const uint64_t deg = p < n ? ecount[p] : 0;
     if (p < n) lsize[p] = deg * ((deg + 63) >> 6);
-    const unsigned w = __reduce_max_sync(kFull, (unsigned)min(deg, (uint64_t)0xffffffffu));
+    const unsigned w = __reduce_max_sync(kFull, (unsigned)deg);
     if ((threadIdx.x & 31) == 0) m[threadIdx.x >> 5] = w;
     __syncthreads();
     if (threadIdx.x) return;
@@ -1710,18 +1713,6 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
     }
 }
 
-// Early-refutation counts and verify-mode counts of an accepted enumeration
-// chunk into the pass's counters.
-__global__ void k_add_tally(const unsigned long long *chunk, unsigned long long *pass) {
-    const int k = threadIdx.x;
-    int which = -1;
-    if (k == 0) which = C_KILLED;
-    else if (k == 1) which = C_KTESTS;
-    else if (k == 2) which = C_CERT;
-    else if (k == 3) which = C_CERT_BAD;
-    if (which >= 0 && chunk[which]) pass[which] += chunk[which];
-}
-
 constexpr int kScanStep = 4;
 constexpr int kScanRefill = 16;  // idle lanes that trigger a refill
 
@@ -1738,12 +1729,17 @@ constexpr int kScanRefill = 16;  // idle lanes that trigger a refill
 // arithmetic; A.verify replays every certified decision too and counts
 // disagreements (C_CERT_BAD).  Survivors are recorded and mark their faces.
 template <int V>
-__global__ void __launch_bounds__(256, V == pac::kExact ? 3 : 4) k_tets_scan(TetArgs A, TetQueue Q, uint64_t nq,
-                                                      unsigned long long *claim) {
+__global__ void __launch_bounds__(256, V == pac::kExact ? 3 : 4) k_tets_scan(TetArgs A, TetQueue Q, const unsigned long long *queued,
+                                                      uint64_t limit, unsigned long long *claim) {
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1;
     unsigned long long evals = 0, oob = 0, certd = 0, bad = 0;
     uint32_t late_alpha = 0, late_killed = 0;  // alpha tests left open by the enumeration
+    const uint64_t nq = *queued;
+    if (nq > limit) return;  // launched ahead of the count: the host sees to it
+    // claims no larger than an equal share: a short queue occupies every warp
+    const unsigned share = (unsigned)min(nq / (8ull * gridDim.x), (unsigned long long)A.scan_claim);
+    const unsigned claim_size = max(32u, share);
     Tally tally;
     uint64_t head = 0, tail = 0;  // this warp's claimed range (warp-uniform)
     bool have = false, more = true;
@@ -1763,10 +1759,10 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 3 : 4) k_tets_scan(Tet
         if (!(__popc(want) >= kScanRefill || want == kFull)) want = 0u;
         if (want && head >= tail && more) {
             uint64_t b = 0;
-            if (lane == 0) b = atomicAdd(claim, (unsigned long long)A.scan_claim);
+            if (lane == 0) b = atomicAdd(claim, (unsigned long long)claim_size);
             b = __shfl_sync(kFull, b, 0);
             head = b;
-            tail = min(nq, b + (uint64_t)A.scan_claim);
+            tail = min(nq, b + (uint64_t)claim_size);
             if (head >= tail) more = false;
             for (uint64_t k = head + 16 * lane; k < tail; k += 512)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(Q.ent + k));
@@ -2532,7 +2528,7 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         CK(cudaMemcpyAsync(mm, init.data(), sizeof(int) * init.size(), cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(d_off, in.h_offsets, sizeof(uint64_t) * (nm + 1),
                            cudaMemcpyHostToDevice, s));
-        CK(cudaStreamSynchronize(s));  // `init` leaves scope
+        // (pageable sources are staged before the calls return)
     }
     if (nm > 1) {
         mol = ar.alloc_n<uint32_t>(n);
@@ -2540,13 +2536,16 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         k_mol_ids<<<nm, 256, 0, s>>>(d_off, nm, mol);
         LAUNCH_CHECK(ctx);
     }
-    k_bbox<<<blocks_for(n, 256), 256, 0, s>>>(in.d_balls, n, mol, mm);
+    k_bbox<<<blocks_for(n, 256), 256, 0, s>>>(in.d_balls, n, mol, mm, ctr);
     LAUNCH_CHECK(ctx);
     k_grid<<<blocks_for(nm, 128), 128, 0, s>>>(mm, nm, in.sol, in.alpha, grids, ncell_d);
     LAUNCH_CHECK(ctx);
     std::vector<MolGrid> hg(nm);
+    unsigned long long bad = 0;
     CK(cudaMemcpyAsync(hg.data(), grids, sizeof(MolGrid) * nm, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(&bad, ctr + C_NONFINITE, sizeof(bad), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    if (bad) return pac::set_error(PAC_ERR_INVALID_ARG, "non-finite ball coordinate or radius");
     uint64_t total_cells = 0;
     for (uint32_t m = 0; m < nm; m++) {
         if (hg[m].gx <= 0 || hg[m].gy <= 0 || hg[m].gz <= 0 || hg[m].ncell > 0x7fffffffull)
@@ -2638,23 +2637,15 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
     LAUNCH_CHECK(ctx);
     rc = exclusive_scan(ctx, ecount, n, eoff);
     if (rc) return rc;
-    uint64_t nE = 0;
-    CK(cudaMemcpyAsync(&nE, eoff + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    uint32_t *ER = ar.alloc_n<uint32_t>(nE);
-    uint8_t *eflag = ar.alloc_n<uint8_t>(nE);
     uint64_t *lsize = ar.alloc_n<uint64_t>(n), *loff = ar.alloc_n<uint64_t>(n + 1);
-    if (!ER || !eflag || !lsize || !loff) return PAC_ERR_OOM;
-    k_edges<V, true><<<warp_blocks(n), 256, 0, s>>>(n, at, cellof, cellbeg, mol, grids, in.alpha,
-                                                    nullptr, eoff, ER, ctr);
-    LAUNCH_CHECK(ctx);
-    CK(cudaMemsetAsync(eflag, 0, nE ? nE : 1, s));
-    k_link_size<<<blocks_for(n, 256), 256, 0, s>>>(n, eoff, lsize, ctr);
+    if (!lsize || !loff) return PAC_ERR_OOM;
+    k_link_size<<<blocks_for(n, 256), 256, 0, s>>>(n, ecount, lsize, ctr);
     LAUNCH_CHECK(ctx);
     rc = exclusive_scan(ctx, lsize, n, loff);
     if (rc) return rc;
-    uint64_t nL = 0;
+    uint64_t nE = 0, nL = 0;
     unsigned long long maxdeg = 0;
+    CK(cudaMemcpyAsync(&nE, eoff + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(&nL, loff + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(&maxdeg, ctr + C_MAXDEG, sizeof(maxdeg), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -2662,6 +2653,13 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         return pac::set_error(PAC_ERR_CAPACITY, "a ball has " + std::to_string(maxdeg) +
                                                     " alpha edges to higher balls; the limit is " +
                                                     std::to_string(kMaxDeg));
+    uint32_t *ER = ar.alloc_n<uint32_t>(nE);
+    uint8_t *eflag = ar.alloc_n<uint8_t>(nE);
+    if (!ER || !eflag) return PAC_ERR_OOM;
+    k_edges<V, true><<<warp_blocks(n), 256, 0, s>>>(n, at, cellof, cellbeg, mol, grids, in.alpha,
+                                                    nullptr, eoff, ER, ctr);
+    LAUNCH_CHECK(ctx);
+    CK(cudaMemsetAsync(eflag, 0, nE ? nE : 1, s));
     tm.mark();  // 2
 
     // ---- alpha triangles (link matrices)
@@ -2692,11 +2690,13 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
     T.maxlen = ctr + C_MAXLEN;
     T.refute = cfg.refute ? 1 : 0;
     T.verify = cfg.verify ? 1 : 0;
+    T.scan_claim = std::max(32, cfg.scan_claim);
     T.tcount = ar.alloc_n<uint32_t>(n);
     uint64_t *toff = ar.alloc_n<uint64_t>(n + 1);
     if (!T.tcount || !toff) return PAC_ERR_OOM;
-    // the enumeration's counts; the scan adds what was left open to it
-    unsigned long long cand_total = 0, alpha_total = 0;
+    // the accepted enumerations' counts; the scan adds what was left open to it
+    constexpr int kEnumCounts[] = {C_CAND_Q, C_ALPHA_Q, C_KILLED, C_KTESTS, C_CERT, C_CERT_BAD};
+    unsigned long long enum_total[C_NCOUNTERS] = {};
     uint64_t nQ = 0;      // tetrahedra output
     uint64_t nQ_all = 0;  // survivors, a slab's halo included
     uint32_t *tets_sorted = nullptr;
@@ -2721,11 +2721,12 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         TetQueue Q;
         Q.ent = ar.alloc_n<uint2>(qcap);
         Q.cap = qcap;
-        uint64_t scap = std::max<uint64_t>(1024, 16 * n);
+        // (at least what a molecule of some 15,000 balls queues: see `ahead`)
+        uint64_t scap = std::max<uint64_t>(1 << 22, 16 * n);
         T.surv = ar.alloc_n<uint2>(scap);
         T.surv_cap = scap;
-        T.pend = ar.alloc_n<uint2>(scap / 4 + 1024);
-        T.pend_cap = scap / 4 + 1024;
+        T.pend_cap = std::max<uint64_t>(1 << 22, scap / 4);
+        T.pend = ar.alloc_n<uint2>(T.pend_cap);
         unsigned long long *claim = ar.alloc_n<unsigned long long>(1);
         unsigned long long *ctrA = ar.alloc_n<unsigned long long>(C_NCOUNTERS);
         uint32_t *classes = ar.alloc_n<uint32_t>(3 * n);  // the enumeration's classes of balls
@@ -2744,18 +2745,25 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
             if (cudaEventElapsedTime(&f, ctx.ev[14], ctx.ev[15]) == cudaSuccess) ortho_ms += f;
             ortho_pending = false;
         };
+        unsigned long long sp[2] = {0, 0};  // survivors, pending
+        bool scanned = false;               // sp holds the final counts
         uint64_t lo = work_lo, chunk = n;
         {
             // first chunk: the whole range when its queue demand (a few
             // entries per alpha triangle) clearly fits, else a probe of 1/32
             // whose fill sizes the next chunks -- an overflowing chunk is
             // enumerated again, smaller
-            unsigned long long atri = 0;
-            CK(cudaMemcpyAsync(&atri, ctr + C_ALPHA_T, sizeof(atri), cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-            // (about 0.5 entries per alpha triangle; 5 without refutation)
+            // (about 0.5 entries per alpha triangle; 5 without refutation);
+            // a ball has at most deg^2 / 2 triangles, which settles all but
+            // the largest passes without reading the count back
+            const double per = cfg.refute ? 1.0 : 8.0;
+            unsigned long long atri = nE * maxdeg / 2;
+            if (per * (double)atri > 0.85 * (double)qcap) {
+                CK(cudaMemcpyAsync(&atri, ctr + C_ALPHA_T, sizeof(atri), cudaMemcpyDeviceToHost, s));
+                CK(cudaStreamSynchronize(s));
+            }
             const double span = (double)(own_hi - work_lo), share = span / (double)std::max<uint64_t>(1, n);
-            if ((cfg.refute ? 1.0 : 8.0) * (double)atri * share > 0.85 * (double)qcap)
+            if (per * (double)atri * share > 0.85 * (double)qcap)
                 chunk = std::max<uint64_t>(1, (uint64_t)(span / 32.0));
         }
         // verbose: per-chunk enumeration and scan times
@@ -2774,9 +2782,25 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
                             : enumerate<M>(ctx, cfg, TA, Q, lo, hi, classes, maxdeg);
             if (rc) return rc;
             if (cfg.verbose) CK(cudaEventRecord(vev[1], s));
-            unsigned long long ha[C_NCOUNTERS], used[2];
+            const unsigned scan_grid = 148u * (unsigned)std::max(1, cfg.scan_blocks);
+            auto scan = [&](uint64_t limit) -> int {
+                CK(cudaMemsetAsync(claim, 0, sizeof(unsigned long long), s));
+                CK(cudaEventRecord(ctx.ev[14], s));
+                k_tets_scan<V><<<scan_grid, 256, 0, s>>>(T, Q, ctrA + C_SURV, limit, claim);
+                LAUNCH_CHECK(ctx);
+                CK(cudaEventRecord(ctx.ev[15], s));
+                ortho_pending = true;
+                return PAC_OK;
+            };
+            // one chunk: the scan goes ahead of its queue's count, and does
+            // nothing should that exceed what the lists hold (then it is
+            // launched again below)
+            const uint64_t room = std::min({qcap, T.surv_cap, T.pend_cap});
+            const bool ahead = lo == work_lo && hi == own_hi;
+            if (ahead && (rc = scan(room))) return rc;
+            unsigned long long ha[C_NCOUNTERS];
             CK(cudaMemcpyAsync(ha, ctrA, sizeof(ha), cudaMemcpyDeviceToHost, s));
-            CK(cudaMemcpyAsync(used, ctr + C_SURV, sizeof(used), cudaMemcpyDeviceToHost, s));
+            CK(cudaMemcpyAsync(sp, ctr + C_SURV, sizeof(sp), cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));
             ortho_collect();
             const unsigned long long queued = ha[C_SURV];
@@ -2787,46 +2811,26 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
                 chunk = std::max<uint64_t>(1, (uint64_t)((double)(hi - lo) * 0.5));
                 continue;
             }
-            // every queued tetrahedron becomes at most one survivor or one
-            // pending entry: grow either list (keeping its entries) first
-            if (used[0] + queued > T.surv_cap) {
-                const uint64_t nc = std::max<uint64_t>(2 * T.surv_cap, used[0] + queued);
-                uint2 *nb = ar.alloc_n<uint2>(nc);
-                if (!nb) return PAC_ERR_OOM;
-                if (used[0])
-                    CK(cudaMemcpyAsync(nb, T.surv, sizeof(uint2) * used[0],
-                                       cudaMemcpyDeviceToDevice, s));
-                T.surv = nb;
-                T.surv_cap = nc;
-            }
-            if (used[1] + queued > T.pend_cap) {
-                const uint64_t nc = std::max<uint64_t>(2 * T.pend_cap, used[1] + queued);
-                uint2 *nb = ar.alloc_n<uint2>(nc);
-                if (!nb) return PAC_ERR_OOM;
-                if (used[1])
-                    CK(cudaMemcpyAsync(nb, T.pend, sizeof(uint2) * used[1],
-                                       cudaMemcpyDeviceToDevice, s));
-                T.pend = nb;
-                T.pend_cap = nc;
-            }
-            cand_total += ha[C_CAND_Q];
-            alpha_total += ha[C_ALPHA_Q];
-            if (ha[C_KILLED] || ha[C_KTESTS] || ha[C_CERT]) {
-                k_add_tally<<<1, 32, 0, s>>>(ctrA, ctr);
-                LAUNCH_CHECK(ctx);
-            }
-            CK(cudaMemsetAsync(claim, 0, sizeof(unsigned long long), s));
-            if (queued) {
-                CK(cudaEventRecord(ctx.ev[14], s));
-                // claims no larger than an equal share: a short queue occupies
-                // every warp
-                const unsigned grid = 148u * (unsigned)std::max(1, cfg.scan_blocks);
-                T.scan_claim = (int)std::min<uint64_t>(std::max(32, cfg.scan_claim),
-                                                       std::max<uint64_t>(32, queued / (8ull * grid)));
-                k_tets_scan<V><<<grid, 256, 0, s>>>(T, Q, queued, claim);
-                LAUNCH_CHECK(ctx);
-                CK(cudaEventRecord(ctx.ev[15], s));
-                ortho_pending = true;
+            for (int k : kEnumCounts) enum_total[k] += ha[k];
+            scanned = ahead && queued <= room;
+            if (!scanned) {
+                // every queued tetrahedron becomes at most one survivor or
+                // one pending entry: grow either list (keeping its entries)
+                // first
+                auto grow = [&](uint2 *&list, uint64_t &cap, unsigned long long used) -> int {
+                    if (used + queued <= cap) return PAC_OK;
+                    const uint64_t nc = std::max<uint64_t>(2 * cap, used + queued);
+                    uint2 *nb = ar.alloc_n<uint2>(nc);
+                    if (!nb) return PAC_ERR_OOM;
+                    if (used)
+                        CK(cudaMemcpyAsync(nb, list, sizeof(uint2) * used, cudaMemcpyDeviceToDevice, s));
+                    list = nb;
+                    cap = nc;
+                    return PAC_OK;
+                };
+                if ((rc = grow(T.surv, T.surv_cap, sp[0]))) return rc;
+                if ((rc = grow(T.pend, T.pend_cap, sp[1]))) return rc;
+                if (queued && (rc = scan(qcap))) return rc;
             }
             if (cfg.verbose) {
                 float me = 0.f, ms = 0.f;
@@ -2853,10 +2857,11 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         }
         if (cfg.verbose)
             for (auto &e : vev) cudaEventDestroy(e);
-        unsigned long long sp[2];
-        CK(cudaMemcpyAsync(sp, ctr + C_SURV, sizeof(sp), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        ortho_collect();
+        if (!scanned) {
+            CK(cudaMemcpyAsync(sp, ctr + C_SURV, sizeof(sp), cudaMemcpyDeviceToHost, s));
+            CK(cudaStreamSynchronize(s));
+            ortho_collect();
+        }
         if (sp[0] > T.surv_cap || sp[1] > T.pend_cap)
             return pac::set_error(PAC_ERR_CAPACITY, "tetrahedron survivor buffer overflow");
         if (sp[1] && sp[0] + sp[1] > T.surv_cap) {  // resolved entries join the survivors
@@ -2933,16 +2938,24 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         CK(cudaMemsetAsync(tricount + work_lo, 0, sizeof(uint32_t) * (own_lo - work_lo), s));
     rc = exclusive_scan(ctx, tricount, n, tpos);
     if (rc) return rc;
-    uint64_t nT = 0;
-    CK(cudaMemcpyAsync(&nT, tpos + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    out.d_tris = ar.alloc_n<uint32_t>(3 * nT);
-    if (!out.d_tris) return PAC_ERR_OOM;
-    k_emit_tris<<<warp_blocks(own_hi - own_lo), 256, 0, s>>>(own_lo, own_hi, eoff, ER, loff, faces,
-                                                            tpos, orig, out.d_tris);
-    LAUNCH_CHECK(ctx);
-    if (in.to_host && (rc = pac::list_to_host_async(ctx, 1, out.d_tris, 3 * nT, &out.h_tris)))
-        return rc;
+    uint64_t nT = 0, nEf = 0;
+    auto emit_tris = [&]() -> int {
+        out.d_tris = ar.alloc_n<uint32_t>(3 * nT);
+        if (!out.d_tris) return PAC_ERR_OOM;
+        k_emit_tris<<<warp_blocks(own_hi - own_lo), 256, 0, s>>>(own_lo, own_hi, eoff, ER, loff, faces,
+                                                                tpos, orig, out.d_tris);
+        LAUNCH_CHECK(ctx);
+        return in.to_host ? pac::list_to_host_async(ctx, 1, out.d_tris, 3 * nT, &out.h_tris) : PAC_OK;
+    };
+    // the triangles leave before the edges are decided, except in passes of a
+    // few thousand balls, where waiting for their count costs more than the
+    // copy takes
+    const bool early = nE > (1u << 20);
+    if (early) {
+        CK(cudaMemcpyAsync(&nT, tpos + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        if ((rc = emit_tris())) return rc;
+    }
     tm.mark();  // 7
 
     // ---- final edges
@@ -2962,9 +2975,14 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
     tm.mark();  // 8
     rc = exclusive_scan(ctx, eflag, nE, epos);
     if (rc) return rc;
-    uint64_t nEf = 0;
+    // every decision is made: the counters and the remaining lengths
+    unsigned long long hc[C_NCOUNTERS];
+    CK(cudaMemcpyAsync(hc, ctr, sizeof(hc), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(&nT, tpos + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(&nEf, epos + nE, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    for (int k : kEnumCounts) hc[k] += enum_total[k];
+    if (!early && (rc = emit_tris())) return rc;
     out.d_edges = ar.alloc_n<uint32_t>(2 * nEf);
     if (!out.d_edges) return PAC_ERR_OOM;
     k_emit_edges<<<warp_blocks(n), 256, 0, s>>>(n, eoff, ER, eflag, epos, orig, out.d_edges);
@@ -2988,24 +3006,18 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         k_mol_rows<<<blocks_for(nm + 1, 128), 128, 0, s>>>(nm, d_off, n, eoff, epos, tpos, toff,
                                                           rows);
         LAUNCH_CHECK(ctx);
-        std::vector<uint64_t> h(3 * (size_t)(nm + 1));
-        CK(cudaMemcpyAsync(h.data(), rows, sizeof(uint64_t) * h.size(), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        for (uint32_t m = 0; m <= nm; m++) {
-            out.edge_off[m] = h[m];
-            out.tri_off[m] = h[(nm + 1) + m];
-            out.tet_off[m] = h[2 * (nm + 1) + m];
-        }
+        CK(cudaMemcpyAsync(out.edge_off.data(), rows, sizeof(uint64_t) * (nm + 1),
+                           cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(out.tri_off.data(), rows + (nm + 1), sizeof(uint64_t) * (nm + 1),
+                           cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(out.tet_off.data(), rows + 2 * (size_t)(nm + 1), sizeof(uint64_t) * (nm + 1),
+                           cudaMemcpyDeviceToHost, s));
     }
     tm.mark();  // 9
     // the lists' copies that did not finish under the later stages
     if (in.to_host && (rc = pac::copies_join(ctx))) return rc;
     tm.mark();  // 10
-    unsigned long long hc[C_NCOUNTERS];
-    CK(cudaMemcpyAsync(hc, ctr, sizeof(hc), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    hc[C_CAND_Q] += cand_total;
-    hc[C_ALPHA_Q] += alpha_total;
     if (hc[C_SOS_RANGE])
         return pac::set_error(PAC_ERR_EXACT_RANGE,
                               "coordinate range too wide for the exact SoS integers");
