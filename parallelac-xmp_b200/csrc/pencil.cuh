@@ -67,6 +67,20 @@
 //    too large for that, or C makes it costly, the caller checks that y lies
 //    within 0.86 steps of X~ on every axis (violators are within R, about 0.8
 //    steps), and hmin leaves 0.125 steps for e / |h| and the rounding of that check.
+//  * Attachment of the triangle itself.  markRealTriangles' centre Xt^ (upstream
+//    formulas) is Cramer's rule over p - v2, v2 - v3 and the computed normal n^,
+//    b3 = n^ . p; checkDanglingTris compares, for a ball e,
+//    |e - Xt^|^2 - w_e with |p - Xt^|^2 - w_p, which differ by s(e) - 2 e' . (Xt^ - p),
+//    and 2 (Xt~ - p) = Q~.  Counting as above (the third row has length N, the
+//    determinant is N^2, a tilt of n^ by 3.6 u |A| |B| / N moves Xt^ along n by
+//    that times |Q| / 2),
+//      |Xt^ - Xt~| <= d = u (65 l C + 16 W L + 26 l R + 3.7 L^2 R) / N + 1.05 u (C + R)
+//    (with contraction + u C^2 L / N), so e attaches the triangle in binary32 when
+//    s(e) - Q~ . e' = g~(e) + (s(e) - s~(e)) < -mt, mt the sum of 2 L d, Eg and the
+//    rounding of the two powers.  Such a ball lies within 1.005 R of Xt (rho <= alpha + 0.01 R^2 is
+//    checked), hence in the window of Xt^ when 1.01 R + 2.1 u C^2 L / N + d is
+//    below 0.99 step; where C or R make that costly, the caller checks that e lies
+//    within 0.95 steps of Xt~ on every axis, and d stays below 0.04 steps.
 // So every bound is affine in N and l with coefficients that depend on the
 // ball p alone.  They are evaluated in binary32 with factors that cover their
 // own rounding; NaN and overflow compare false, so nothing is certified then.
@@ -92,16 +106,20 @@ struct Bounds {
     float m4[3];      // alpha test, times |n|^2
     float hmin[3];
     float nmin2;      // |n|^2 below this: needle triangles (double's rounding of n would show)
+    float mt[3];      // attachment: (mt[0] + mt[1] l) / N + mt[2]
+    float mw, mtmax;  // its use needs mw / N + mt < mtmax
+    float mreach;     // 0.95 step where its window needs the check by distance, else 0
+    float base4;      // 4 (w + alpha) + 0.04 R^2
     float kappa;      // the alpha test's limit in |h| is kappa hmin
     float q2max;      // |Q|^2 above this certifies nothing
     float alpha;
     float reach;      // 0.86 step where the window needs the check by distance, else 0
 };
 
-// maxlen2: largest squared length of an alpha edge (binary32); wmax: upper
+// p's centre and weight; maxlen2: largest squared length of an alpha edge (binary32); wmax: upper
 // bound of every weight; contracted: markRealTets compiled with FMA contraction.
-PAC_PENCIL_FN Bounds bounds(float px, float py, float pz, float alpha, float maxlen2, float wmax,
-                            float step, bool contracted) {
+PAC_PENCIL_FN Bounds bounds(float px, float py, float pz, float wp, float alpha, float maxlen2,
+                            float wmax, float step, bool contracted) {
     Bounds b;
     const float L = sqrtf(maxlen2) * 1.001f, L2 = L * L, W = wmax;
     const float R = sqrtf(fmaxf(W + alpha, 0.0f)) * 1.001f, R2 = R * R;
@@ -138,6 +156,16 @@ PAC_PENCIL_FN Bounds bounds(float px, float py, float pz, float alpha, float max
     const float a2 = 1.02f * (1024.0f * 14.0f * kU * L + 9.0f * iR * eb + iR2 * b.m4[2]);
     b.kappa = 1.0001f * fmaxf(fmaxf(1.0f, a0 / b.hmin[0]), fmaxf(a1 / b.hmin[1], a2 / b.hmin[2]));
     b.alpha = alpha;
+    const float ct = contracted ? 1.05f * kU * C * C * L : 0.0f;
+    b.mt[0] = 1.02f * 2.0f * L * (kU * (16.0f * W * L + 3.7f * L2 * R) + ct);
+    b.mt[1] = 1.02f * kU * 2.0f * L * (65.0f * C + 26.0f * R);
+    b.mt[2] = 1.02f * (kU * (2.1f * L * (C + R) + 16.0f * (2.0f * R2 + W)) + Eg) + 1e-20f;
+    const float aslack = 0.99f * step - 1.01f * R;
+    const bool near_ok = aslack > 0.02f * R && 10.0f * kU * C * C < 0.3f * aslack * L;
+    b.mreach = near_ok ? 0.0f : 0.95f * step;
+    b.mw = near_ok ? 2.2f * kU * C * C * L * 2.0f * L : 0.0f;
+    b.mtmax = 2.0f * L * (near_ok ? aslack : 0.04f * step);
+    b.base4 = 4.0f * (wp + alpha) + 0.04f * R2;
     b.nmin2 = fmaxf(1e-6f * L2 * L2, 1e-18f);
     b.q2max = 4.1f * R2;
     // sizes the bounds were not written for certify nothing
@@ -150,6 +178,7 @@ struct Group {
     float qx, qy, qz, rg;    // Q, the refutation's margin
     float tx, ty, tz, k;     // Q~, the alpha test's k
     float ea;                // and margin
+    float mt;                // attachment's margin
 };
 
 // A neighbour of p: its position relative to p, its lift s and the lift s~ of
@@ -189,8 +218,10 @@ PAC_PENCIL_FN Group group(const Bounds &b, const Point &A, const Point &B, float
     g.ea = fmaf(b.m4[1], N, fmaf(b.m4[2], l, b.m4[0])) * inv;
     g.k = 4.0f * (b.alpha - base) * inv;
     const float hm = fmaf(b.hmin[1], N, fmaf(b.hmin[2], l, b.hmin[0]));
+    const float mt = fmaf(fmaf(b.mt[1], l, b.mt[0]), N * inv, b.mt[2]);
     const bool fine = N2 > b.nmin2 && q2 < b.q2max && hm < 1e18f;
     g.hmin = fine ? hm : INFINITY;
+    g.mt = fine && q2 < b.base4 && fmaf(b.mw, N * inv, mt) < b.mtmax ? mt : INFINITY;
     return g;
 }
 
@@ -199,6 +230,12 @@ PAC_PENCIL_FN float height(float nx, float ny, float nz, float x, float y, float
 }
 PAC_PENCIL_FN float power(float qx, float qy, float qz, float s, float x, float y, float z) {
     return fmaf(-qz, z, fmaf(-qy, y, fmaf(-qx, x, s)));
+}
+
+// Whether z lies within reach, per axis, of the triangle's centre Xt~.
+PAC_PENCIL_FN bool in_box(float tx, float ty, float tz, float x, float y, float z, float reach) {
+    return fmaxf(fabsf(fmaf(-0.5f, tx, x)),
+                 fmaxf(fabsf(fmaf(-0.5f, ty, y)), fabsf(fmaf(-0.5f, tz, z)))) <= reach;
 }
 
 // Alpha test of x (a = |h(x)| >= kappa hmin, gt = g~(x)): certainly alpha, certainly

@@ -816,6 +816,8 @@ struct TetArgs {
     uint32_t *tets_out;   // as-run fill: sorted-space vertex quadruples
     unsigned long long *ctr;   // the pass's counters, or a chunk's (enumeration)
     const unsigned long long *maxlen;  // C_MAXLEN of the pass
+    uint64_t *attached;        // enumeration: alpha triangles a neighbour attaches (shape of
+                               // link), or null
     int refute;                // enumeration: refute early against the group's firsts
     int verify;                // scan: replay every certified decision and count disagreements
     int scan_claim;            // queue entries a scan warp claims at a time
@@ -1142,7 +1144,7 @@ struct GroupRec {
     float4 qe;       // Q, ea
     float4 tk;       // Q~, k
     float rg;
-    uint32_t ab;     // a | b << 8
+    uint32_t ab;     // a | b << 8 | attachment margin (16 bits); the sign: found attached
     uint32_t best[2];  // per side: pencil position (24 bits) | c of its first; then c | (refuted) << 8
     float2 first[2]; // h, g of the firsts
 };
@@ -1152,7 +1154,7 @@ static_assert(sizeof(GroupRec) == 80, "bank layout");
 template <int KW>
 struct EnumSmem {
     static constexpr int kDeg = 64 * KW, kTab = KW == 1 ? 1024 : KW == 2 ? 2048 : 8192;
-    static constexpr int kSlots = KW == 1 ? 224 : 256;  // candidates at a time (one group has fewer)
+    static constexpr int kSlots = KW == 1 ? 216 : 256;  // candidates at a time (one group has fewer)
     static constexpr int kWords = 2 * KW;
     static constexpr int kGroups = 1024;  // triangles listed at a time (one row has fewer)
     static constexpr int kWarps = KW == 1 ? 4 : KW == 2 ? 12 : 16;
@@ -1169,6 +1171,7 @@ struct EnumSmem {
     uint16_t cand[kWarps][kSlots];  // listed candidates: group | c << 5 | kCand* bits
     float st[kDeg];              // lifts of the rounded squares
     uint32_t sN[kDeg];           // upper neighbours
+    uint32_t att[kDeg * kWords]; // triangles found attached: bits b of row a
     uint32_t rowpre[kDeg + 1];   // triangles with fourth vertices before each row
     uint32_t next, chunk;        // the block's ball, its next chunk
     uint16_t tri[kGroups];       // p's triangles: a | b << 8
@@ -1232,10 +1235,13 @@ __device__ __forceinline__ void queue_close(const TetQueue &Q, QRes &qr) {
 // The balls of [lo, hi) by class (at most 64, 128, 256 upper neighbours; at
 // least 3): list[class * n ..], counted in ctr[C_CLASS + class].
 __global__ void k_classes(uint64_t lo, uint64_t hi, uint64_t n, const uint64_t *eoff,
-                          uint32_t *list, unsigned long long *ctr) {
+                          const uint64_t *loff, uint64_t *attached, uint32_t *list,
+                          unsigned long long *ctr) {
     const uint64_t p = lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const int deg = p < hi ? (int)(eoff[p + 1] - eoff[p]) : 0;
+    if (attached && deg > 0 && deg < 3)  // no class: its rows are not written there
+        for (int a = 0; a < deg; a++) attached[loff[p] + a] = 0;
     const int mine = deg < 3 ? -1 : deg <= 64 ? 0 : deg <= 128 ? 1 : 2;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
@@ -1298,6 +1304,23 @@ __device__ __noinline__ void enum_verify(const TetArgs &A, const MolGrid &G, con
     }
 }
 
+// Verify mode: a certified attachment of the triangle by ball e.
+template <int M>
+__device__ __noinline__ void attach_verify(const TetArgs &A, const MolGrid &G, const float4 b1,
+                                           const float4 b2, const float4 b3, const float4 e) {
+    constexpr int V = (M & kEnumExact) ? pac::kExact : pac::kUpstream;
+    Tally tally;
+    const Ball B1{b1.x, b1.y, b1.z, b1.w}, B2{b2.x, b2.y, b2.z, b2.w}, B3{b3.x, b3.y, b3.z, b3.w},
+        E{e.x, e.y, e.z, e.w};
+    const float4 o = tri_sphere<V>(B1, B2, B3, A.alpha);
+    bool att;
+    if constexpr (V == pac::kExact) att = pac::ex::tri_attached(B1, B2, B3, E, tally);
+    else att = pac::attached(E, o.x, o.y, o.z, o.w);
+    atomicAdd(&A.ctr[C_CERT], 1ull);
+    if (!att || !surely_in_window(o.x, o.y, o.z, e.x, e.y, e.z, 0.99f * G.step))
+        atomicAdd(&A.ctr[C_CERT_BAD], 1ull);
+}
+
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -1354,6 +1377,8 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
         __syncthreads();
         const uint32_t p = S.next;
         if (p == kNoTet) break;
+        // (each thread clears what it wrote out for the previous ball)
+        for (int k = tid; k < Smem::kDeg * KW; k += kThreads) *(uint64_t *)&S.att[2 * k] = 0;
         const uint64_t e0 = A.eoff[p];
         const int deg = (int)(A.eoff[p + 1] - e0);
         const MolGrid &G = A.grids[mol_of(A.mol, p)];
@@ -1361,7 +1386,7 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
         const float w1 = __fmul_rn(b1.w, b1.w);  // (its rounding in the exact mode is inside the bounds)
         const bool refute = A.refute && G.gx <= 16384 && G.gy <= 16384 && G.gz <= 16384;
         if (tid == 0)
-            S.bounds = pac::pencil::bounds(b1.x, b1.y, b1.z, A.alpha,
+            S.bounds = pac::pencil::bounds(b1.x, b1.y, b1.z, w1, A.alpha,
                                            __uint_as_float((uint32_t)*A.maxlen), G.wmax, G.step,
                                            kContracted);
         // ---- the ball's neighbours, relative to it, and its link rows
@@ -1455,7 +1480,7 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
         }
         __syncthreads();
         const bool slow = S.bounds.reach > 0.f || (M & kEnumVerify);
-        const float kappa = S.bounds.kappa;
+        const float kappa = S.bounds.kappa, mreach = S.bounds.mreach;
         // ---- the triangles (p, N[a], N[b]): rows [row0, row1) listed at a
         // time, 32 triangles per chunk
         for (int row0 = 0, row1; row0 < deg; row0 = row1) {
@@ -1523,7 +1548,10 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
                 R.qe = make_float4(gr.qx, gr.qy, gr.qz, gr.ea);
                 R.tk = make_float4(gr.tx, gr.ty, gr.tz, gr.k);
                 R.rg = gr.rg;
-                R.ab = (uint32_t)a | ((uint32_t)b << 8);
+                // the attachment margin rounded up to 16 bits
+                const float mt = A.attached ? gr.mt : INFINITY;
+                R.ab = (uint32_t)a | ((uint32_t)b << 8) |
+                       (min(__float_as_uint(mt) + 0xffffu, 0x7f800000u) & 0xffff0000u);
                 R.best[0] = R.best[1] = 0xffffffffu;
                 S.face[wib][0][r] = (uint32_t)f0;
                 S.face[wib][1][r] = (uint32_t)(f0 >> 32);
@@ -1576,12 +1604,12 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
                     bits &= bits - 1;
                     GroupRec &R = S.group[wib][j];
                     const uint32_t ab = R.ab;
-                    const uint32_t mc = S.map[ab & 0xff][c];
+                    const uint32_t a = ab & 0xff, b = (ab >> 8) & 0xff;
+                    const uint32_t mc = S.map[a][c];
                     uint32_t row = S.face[wib][(mc >> 5) & 3][j];
-                    if (wide && act && S.d2[ab & 0xff] > 128)
-                        row = ((const uint32_t *)&A.link[S.l2[ab & 0xff] +
-                                                         (uint64_t)S.map[ab & 0xff][ab >> 8] *
-                                                             ((S.d2[ab & 0xff] + 63) >> 6)])[mc >> 5];
+                    if (wide && act && S.d2[a] > 128)
+                        row = ((const uint32_t *)&A.link[S.l2[a] + (uint64_t)S.map[a][b] *
+                                                                       ((S.d2[a] + 63) >> 6)])[mc >> 5];
                     const bool face = act && ((row >> (mc & 31)) & 1u);
                     const float4 z = S.rel[c], nh = R.nh, qe = R.qe, tk = R.tk;
                     const float h = pac::pencil::height(nh.x, nh.y, nh.z, z.x, z.y, z.z);
@@ -1589,6 +1617,15 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
                     const float gt = kPerturbed
                                          ? pac::pencil::power(tk.x, tk.y, tk.z, S.st[c], z.x, z.y, z.z)
                                          : q;
+                    // does this neighbour attach the triangle?  One or
+                    // another does for most, at a few operations here;
+                    // k_tri_attach tests the other triangles
+                    if (gt + (z.w - S.st[c]) < -fabsf(__uint_as_float(ab & 0xffff0000u)) && act &&
+                        (mreach == 0.f || pac::pencil::in_box(tk.x, tk.y, tk.z, z.x, z.y, z.z, mreach))) {
+                        R.ab = ab | 0x80000000u;
+                        if constexpr (M & kEnumVerify)
+                            attach_verify<M>(A, G, b1, A.at[S.sN[a]], A.at[S.sN[b]], A.at[S.sN[c]]);
+                    }
                     const float a0 = fabsf(h);
                     const bool sure = a0 >= nh.w;
                     bool in, out;
@@ -1603,8 +1640,8 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
                     open_acc += open;
                     if constexpr (M & kEnumVerify)
                         if (face)
-                            enum_verify<M>(A, G, b1, A.at[S.sN[ab & 0xff]], A.at[S.sN[ab >> 8]],
-                                           A.at[S.sN[c]], in ? 1 : out ? 0 : -1, nullptr);
+                            enum_verify<M>(A, G, b1, A.at[S.sN[a]], A.at[S.sN[b]], A.at[S.sN[c]], in ? 1 : out ? 0 : -1,
+                                           nullptr);
                     const unsigned m = __ballot_sync(kFull, live);
                     if (live) {
                         const int at = n + __popc(m & lt_mask);
@@ -1635,6 +1672,7 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
                     }
                     // (0 when either side is empty: nothing refuted)
                     const uint32_t both = pac::pencil::refutes(h0, q0, h1, q1, R.rg) ? 256u : 0u;
+                    if (R.ab >> 31) atomicOr(&S.att[a * Smem::kWords + (b >> 5)], 1u << (b & 31));
                     R.first[0] = make_float2(h0, q0);
                     R.first[1] = make_float2(h1, q1);
                     R.best[0] = (uint32_t)y0 | both;
@@ -1668,12 +1706,12 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
                                 if constexpr (M & kEnumVerify)
                                     if (dead)
                                         enum_verify<M>(A, G, b1, A.at[S.sN[R.ab & 0xff]],
-                                                       A.at[S.sN[R.ab >> 8]], A.at[S.sN[c]],
+                                                       A.at[S.sN[(R.ab >> 8) & 0xff]], A.at[S.sN[c]],
                                                        -1, &A.at[S.sN[v]]);
                             }
                             take = !dead || (e & kCandOpen);
                             if (take)
-                                key = R.ab | ((uint32_t)c << 16) |
+                                key = (R.ab & 0xffffu) | ((uint32_t)c << 16) |
                                       (e & kCandOpen ? kAlphaOpen : 0u) | (dead ? kRefuted : 0u);
                         }
                         const unsigned m = __ballot_sync(kFull, take);
@@ -1691,6 +1729,12 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
             if (tid == 0) S.chunk = 0;
             __syncthreads();
         }
+        }
+        if (A.attached) {
+            const int W = (deg + 63) >> 6;
+            uint64_t *out = A.attached + A.loff[p];
+            for (int k = tid; k < deg * KW; k += kThreads)
+                if (k % KW < W) out[(uint64_t)(k / KW) * W + k % KW] = *(const uint64_t *)&S.att[2 * k];
         }
         if (qr.wait) {
             __syncwarp();
@@ -2075,7 +2119,7 @@ __global__ void k_map4(uint64_t nq, const uint32_t *orig, uint32_t *tets) {
 
 // ------------------------------------------------------------------ attachment
 // Final triangles of ball v1: tetrahedron faces, plus the alpha triangles
-// that are not faces and whose orthosphere no other ball of the 27-cell
+// that are neither faces nor found attached by the enumeration and whose orthosphere no other ball of the 27-cell
 // window reaches (checkDanglingTris, AlphaComplexLargeData.cu:798-872).
 // Work stealing: one warp per ball v1, balls handed out from a counter.  The alpha triangles
 // of v1 that are not tetrahedron faces are queued in shared memory row by
@@ -2094,6 +2138,7 @@ __global__ void __launch_bounds__(256, 4) k_tri_attach(uint64_t p_lo, uint64_t n
                                                        const uint32_t *__restrict__ ER,
                                                        const uint64_t *__restrict__ loff,
                                                        const uint64_t *__restrict__ link,
+                                                       const uint64_t *__restrict__ attached,
                                                        uint64_t *faces, uint32_t *tricount,
                                                        uint8_t *eflag, const uint32_t *cellbeg,
                                                        const uint32_t *mol, const MolGrid *grids,
@@ -2137,9 +2182,11 @@ __global__ void __launch_bounds__(256, 4) k_tri_attach(uint64_t p_lo, uint64_t n
                         if (!rloaded) {
 #pragma unroll
                             for (int w = 0; w < kMaxW; w++)
-                                rbits[w] = w < W ? (link[lp + (uint64_t)row * W + w] &
-                                                    ~faces[lp + (uint64_t)row * W + w])
-                                                 : 0;
+                            {
+                                const uint64_t at = lp + (uint64_t)row * W + w;
+                                rbits[w] = w < W ? (link[at] & ~faces[at]) : 0;
+                                if (attached && w < W) rbits[w] &= ~attached[at];
+                            }
                             rloaded = true;
                         }
                         int nc = 0;
@@ -2447,7 +2494,8 @@ static int enumerate(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const TetArg
     int rc = enum_smem_optin<M>(ctx);
     if (rc) return rc;
     const uint64_t balls = hi - lo;
-    k_classes<<<(unsigned)((balls + 255) / 256), 256, 0, s>>>(lo, hi, A.n, A.eoff, list, A.ctr);
+    k_classes<<<(unsigned)((balls + 255) / 256), 256, 0, s>>>(lo, hi, A.n, A.eoff, A.loff, A.attached, list,
+                                                               A.ctr);
     LAUNCH_CHECK(ctx);
     const unsigned light = (unsigned)std::min<uint64_t>(balls, 148u * (unsigned)std::max(1, cfg.enum_blocks));
     const unsigned heavy = (unsigned)std::min<uint64_t>(balls, 148u * (unsigned)std::max(1, cfg.heavy_blocks));
@@ -2716,6 +2764,15 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         k_tets<V, 2><<<warp_blocks(n), 256, 0, s>>>(T);
         LAUNCH_CHECK(ctx);
     } else {
+        // the enumeration settles most triangle attachments on its way (not
+        // with the plain-xmp formulas, whose triangle centres are no
+        // orthocentres, nor where the window lemma's grid limit is exceeded)
+        bool small_grid = true;
+        for (const MolGrid &g : hg) small_grid &= g.gx <= 16384 && g.gy <= 16384 && g.gz <= 16384;
+        if (V != pac::kPlainXmp && small_grid) {
+            T.attached = ar.alloc_n<uint64_t>(nL);
+            if (!T.attached) return PAC_ERR_OOM;
+        }
         // queue of alpha tetrahedra in HBM, processed in chunks of balls
         const uint64_t qcap = std::max<uint64_t>(1 << 16, cfg.queue_entries);
         TetQueue Q;
@@ -2929,7 +2986,7 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
     CK(cudaMemsetAsync(ctr + C_NEXT, 0, sizeof(unsigned long long), s));
     if (cfg.slab_world > 1) CK(cudaMemsetAsync(tricount, 0, sizeof(uint32_t) * n, s));
     k_tri_attach<V><<<std::min<unsigned>(warp_blocks(own_hi - work_lo), 148 * 4), 256, 0, s>>>(
-        work_lo, own_hi, at, eoff, ER, loff, link, faces, tricount, eflag, cellbeg, mol, grids,
+        work_lo, own_hi, at, eoff, ER, loff, link, T.attached, faces, tricount, eflag, cellbeg, mol, grids,
         in.alpha, ctr);
     LAUNCH_CHECK(ctx);
     tm.mark();  // 6

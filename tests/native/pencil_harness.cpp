@@ -6,7 +6,7 @@
 // flavour the polynomials' exact signs (orc_exact_pred).  Built and run by
 // tests/test_pencil.py.
 //   pencil_harness SEED CLUSTERS OFFSET SOL LATTICE EXACT
-//     -> "alpha N certified C bad B refutations R bad B"
+//     -> "alpha N certified C bad B refutations R bad B attachments A bad B"
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -53,7 +53,7 @@ int main(int argc, char **argv) {
     const int clusters = atoi(argv[2]);
     const double offset = atof(argv[3]), sol = atof(argv[4]);
     const bool lattice = atoi(argv[5]), ex = atoi(argv[6]);
-    long tests = 0, certified = 0, bad = 0, refuted = 0, rbad = 0;
+    long tests = 0, certified = 0, bad = 0, refuted = 0, rbad = 0, attached = 0, abad = 0;
     for (int t = 0; t < clusters; t++) {
         const float alpha = t % 3 == 0 ? 0.0f : t % 3 == 1 ? 0.5f : 1.0f;
         const float step = 2.0f * std::sqrt(1.8f * 1.8f + alpha);
@@ -84,7 +84,7 @@ int main(int argc, char **argv) {
         }
         const Ball &p = b[0];
         const pac::pencil::Bounds bounds =
-            pac::pencil::bounds(p.x, p.y, p.z, alpha, len2, wmax, step, false);
+            pac::pencil::bounds(p.x, p.y, p.z, p.r * p.r, alpha, len2, wmax, step, false);
         const double wp = ex ? (double)p.r * p.r : (double)(p.r * p.r);
         std::vector<pac::pencil::Point> P(n);
         for (int k = 0; k < n; k++) {
@@ -98,6 +98,28 @@ int main(int argc, char **argv) {
             for (int j = i + 1; j < n; j++) {
                 if (!edge[i] || !edge[j] || !edge[i * n + j]) continue;
                 const pac::pencil::Group g = pac::pencil::group(bounds, P[i], P[j], p.r * p.r);
+                // attachment of the triangle by any other neighbour of p
+                float4 to;
+                if (ex ? exact(1, {p, b[i], b[j]}, alpha) != 0
+                       : pac::tri_alpha<pac::kUpstream>(p, b[i], b[j], alpha, to))
+                    for (int v = 1; v < n; v++) {
+                        if (v == i || v == j || !edge[v]) continue;
+                        const float s0 = (float)P[v].s, st = (float)P[v].st, x = (float)P[v].x,
+                                    y = (float)P[v].y, zz = (float)P[v].z;
+                        const float gt = pac::pencil::power(g.tx, g.ty, g.tz, st, x, y, zz);
+                        if (!(gt + (s0 - st) < -g.mt)) continue;
+                        if (bounds.mreach > 0 &&
+                            !pac::pencil::in_box(g.tx, g.ty, g.tz, x, y, zz, bounds.mreach))
+                            continue;
+                        attached++;
+                        if (ex) {
+                            abad += exact(6, {p, b[i], b[j], b[v]}, alpha) == 0;
+                            continue;
+                        }
+                        const float m = std::max(std::fabs(b[v].x - to.x), std::max(std::fabs(b[v].y - to.y),
+                                                                                    std::fabs(b[v].z - to.z)));
+                        abad += !pac::attached(b[v], to.x, to.y, to.z, to.w) || !(m <= 0.99f * step);
+                    }
                 std::vector<int> z;
                 for (int k = 1; k < n; k++)
                     if (k != i && k != j && edge[k] && edge[i * n + k] && edge[j * n + k]) z.push_back(k);
@@ -152,7 +174,7 @@ int main(int argc, char **argv) {
                 }
             }
     }
-    std::printf("alpha %ld certified %ld bad %ld refutations %ld bad %ld\n", tests, certified, bad, refuted,
-                rbad);
+    std::printf("alpha %ld certified %ld bad %ld refutations %ld bad %ld attachments %ld bad %ld\n", tests, certified,
+                bad, refuted, rbad, attached, abad);
     return 0;
 }

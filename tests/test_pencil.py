@@ -34,6 +34,9 @@ def test_pencil_filter_never_disagrees(harness, offset, sol, lattice, exact):
     print(r.stdout.strip())
     tests, cert, bad, refuted, rbad = (int(f[k]) for k in (1, 3, 5, 7, 9))
     assert bad == 0 and rbad == 0
+    attached, abad = int(f[11]), int(f[13])
+    assert abad == 0
+    assert attached > 1000 or sol > 3  # (a window not certain leaves them to the general path)
     assert tests > 1000 and refuted > 1000
     assert cert > (0.5 if offset < 1000 else 0.2) * tests
 
