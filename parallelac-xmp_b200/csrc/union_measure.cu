@@ -254,18 +254,17 @@ __device__ __forceinline__ void dd_add(double &hi, double &lo, double bh, double
     lo = e - (hi - s);
 }
 
-// Sums v over the run of consecutive active lanes with the same id, in lane
-// order; true for the run's first lane, which then holds the sum.  The lists
+// Sums v over the run of consecutive lanes of act (a prefix of the warp, all of
+// which call) with the same id, in lane order; true for the run's first lane, which then holds the sum.  The lists
 // group simplices by their first vertex (in the complex's own order runs of 5
 // to 11), whose atomics, a quarter to a half of all, shrink by that much:
 // 224 us of atomics for 2.3 M simplices without it.
-__device__ __forceinline__ bool run_sum(uint32_t id, double (&v)[8]) {
-    const unsigned act = __activemask();
+__device__ __forceinline__ bool run_sum(unsigned act, uint32_t id, double (&v)[8]) {
     const int lane = threadIdx.x & 31;
     const uint32_t left = __shfl_up_sync(act, id, 1);
     const bool head = lane == 0 || left != id;
     const unsigned heads = __ballot_sync(act, head);
-    // lanes up to the next head (active lanes are a prefix of the warp)
+    // lanes up to the next head
     const unsigned above = lane == 31 ? 0u : heads & (0xfffffffeu << lane);
     const int end = above ? __ffs((int)above) - 1 : __popc(act);
 #pragma unroll
@@ -291,6 +290,7 @@ __global__ void __launch_bounds__(128, K >= 3 ? 4 : 8) k_union(uint64_t ns, cons
     __shared__ double4 wpart[4];
     uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     double vh = 0, vl = 0, ah = 0, al = 0;
+    const unsigned act = __ballot_sync(0xffffffffu, s < ns);
     if (s < ns) {
         uint32_t id[K];
         V3 c[K];
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(128, K >= 3 ? 4 : 8) k_union(uint64_t ns, cons
                                sg * (inv * T.M[q].z + T.rN[q].z), sg * (inv * T.A[q] + T.rl[q])};
                 bool lead = true;
                 if constexpr (K > 1)
-                    if (q == 0) lead = run_sum(id[0], v);
+                    if (q == 0) lead = run_sum(act, id[0], v);
                 if (lead) {
 #pragma unroll
                     for (int t = 0; t < 4; t++) {
