@@ -682,113 +682,216 @@ __global__ void __launch_bounds__(256) k_link_size(uint64_t n, const uint32_t *e
     if (top > *(volatile unsigned long long *)&ctr[C_MAXDEG]) atomicMax(&ctr[C_MAXDEG], (unsigned long long)top);
 }
 
+// The balls of [lo, hi) by class (at most 64, 128, 256 upper neighbours; at
+// least `least`): list[class * n ..], counted in ctr[C_CLASS + class].
+__global__ void k_classes(uint64_t lo, uint64_t hi, uint64_t n, const uint64_t *eoff,
+                          const uint64_t *loff, uint64_t *attached, int least, uint32_t *list,
+                          unsigned long long *ctr) {
+    const uint64_t p = lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const int deg = p < hi ? (int)(eoff[p + 1] - eoff[p]) : 0;
+    if (attached && deg > 0 && deg < 3)  // no class: its rows are not written there
+        for (int a = 0; a < deg; a++) attached[loff[p] + a] = 0;
+    const int mine = deg < least ? -1 : deg <= 64 ? 0 : deg <= 128 ? 1 : 2;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const unsigned m = __ballot_sync(kFull, mine == c);
+        if (!m) continue;
+        unsigned long long b = 0;
+        if (lane == 0) b = atomicAdd(&ctr[C_CLASS + c], (unsigned long long)__popc(m));
+        b = __shfl_sync(kFull, b, 0);
+        if (mine == c) list[c * n + b + __popc(m & ((1u << lane) - 1))] = (uint32_t)p;
+    }
+}
+
 // ------------------------------------------------------------------ triangles
-// One warp per ball i: bit (a, b) of i's link matrix is set when
-// (i, v1 = N[a], v2 = N[b]) is a candidate triangle -- edge v1v2 is an alpha
-// edge (AlphaComplexLargeData.cu:192-296) -- and passes markRealTriangles.
-template <int V>
-__global__ void __launch_bounds__(256) k_link(uint64_t n, const float4 *__restrict__ at,
+// Bit (a, b) of ball i's link matrix is set when (i, v1 = N[a], v2 = N[b]) is a
+// candidate triangle -- edge v1v2 is an alpha edge (AlphaComplexLargeData.cu:
+// 192-296) -- and passes markRealTriangles.  A block per ball of one class (see
+// k_classes).  The edges among a ball's neighbours come from one table look-up
+// per neighbour of a neighbour (a binary search in global memory per pair took
+// half of the time); the candidates are then cut into equal shares over the
+// block's threads, so that every lane evaluates markRealTriangles.
+// What bounds it: instruction issue, most of it markRealTriangles.  A warp per
+// ball searching pair by pair, 21 of 32 lanes: 1.98 ms at 100,000 balls, 105 us
+// at 211.
+
+// Slot of ball x in a table of 2^bits, for attempt t: the neighbours of a ball
+// are a few runs of consecutive indices, which the low bits usually keep apart.
+constexpr int kHashTries = 8;
+__device__ __forceinline__ uint32_t hash_slot(uint32_t x, int t, int bits) {
+    return t == 0 ? x & ((1u << bits) - 1) : (x * (2654435769u * (2u * t + 1u))) >> (32 - bits);
+}
+
+// A table from ball indices to positions in the list ids[0..deg), whose entries
+// are written for attempt 0: tries others until no two of the list collide.
+// Returns the attempt, or kHashTries when all collide (block-uniform; ends
+// with a barrier).
+__device__ __forceinline__ int settle_table(uint8_t *tab, const uint32_t *ids, int deg, int bits) {
+    int tries = 0;
+    while (true) {
+        bool clash = false;
+        for (int c = threadIdx.x; c < deg; c += blockDim.x)
+            clash |= tab[hash_slot(ids[c], tries, bits)] != (uint8_t)c;
+        if (!__syncthreads_or(clash) || ++tries == kHashTries) return tries;
+        for (int c = threadIdx.x; c < deg; c += blockDim.x)
+            tab[hash_slot(ids[c], tries, bits)] = (uint8_t)c;
+        __syncthreads();
+    }
+}
+// The position of x in the list, or some other position (compare ids there):
+// a slot that no listed ball wrote holds anything.  size: of ids' array, a
+// power of two.
+__device__ __forceinline__ int table_find(const uint8_t *tab, const uint32_t *ids, int deg, int size,
+                                          int bits, int tries, uint32_t x) {
+    if (tries < kHashTries) return tab[hash_slot(x, tries, bits)] & (size - 1);
+    int lo = 0, hi = deg;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (ids[mid] <= x) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+template <int KW>
+struct LinkSmem {
+    static constexpr int kDeg = 64 * KW, kBits = KW == 1 ? 10 : KW == 2 ? 11 : 13, kWords = 2 * KW;
+    float4 ball[kDeg];           // the upper neighbours
+    uint64_t e2[kDeg];           // each one's first upper neighbour's index
+    uint32_t edge[kDeg * kWords + 1];  // bits b of row a: alpha edge (N[a], N[b]); all ones at the end
+    uint32_t tri[kDeg * kWords]; // the link rows
+    uint32_t id[kDeg];
+    uint32_t rowpre[kDeg + 1];   // candidates before each row
+    uint32_t next;
+    uint16_t d2[kDeg];           // upper degrees
+    uint8_t tab[1 << kBits];
+};
+
+template <int V, int KW>
+__global__ void __launch_bounds__(128) k_link(const uint32_t *list, int cls,
+                                              const float4 *__restrict__ at,
                                               const uint64_t *__restrict__ eoff,
                                               const uint32_t *__restrict__ ER,
                                               const uint64_t *__restrict__ loff, uint64_t *link,
                                               float alpha, unsigned long long *ctr) {
-    __shared__ uint64_t srow[8][kMaxW];
-    __shared__ uint64_t sL[8][64];  // link rows of a ball of <= 64 upper neighbours
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    unsigned long long cand_acc = 0, alpha_acc = 0;
+    using Smem = LinkSmem<KW>;
+    constexpr int kWords = Smem::kWords, kThreads = 128, kWarps = 4;
+    __shared__ Smem S;
+    const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
+    uint32_t cand_acc = 0, alpha_acc = 0;
     Tally tally;
-    // balls handed out by a counter: a warp that finishes a small ball takes
-    // the next one instead of waiting for its block's largest
-    for (;;) {
-        uint64_t p = 0;
-        if (lane == 0) p = atomicAdd(&ctr[C_NEXT], 1ull);
-        p = __shfl_sync(kFull, p, 0);
-        if (p >= n) break;
+    const uint64_t count = ctr[C_CLASS + cls];
+    while (true) {
+        __syncthreads();  // the previous ball's shared memory is free
+        if (tid == 0) {
+            const unsigned long long u = atomicAdd(&ctr[C_TAKE + cls], 1ull);
+            S.next = u < count ? list[u] : 0xffffffffu;
+        }
+        __syncthreads();
+        const uint32_t p = S.next;
+        if (p == 0xffffffffu) break;
         const uint64_t e0 = eoff[p];
         const int deg = (int)(eoff[p + 1] - e0);
-        if (deg < 2) continue;
-        const int W = (deg + 63) >> 6;
-        const uint32_t *N = ER + e0;
-        uint64_t *L = link + loff[p];
         const Ball A = pac::ld_ball(&at[p]);
-        if (deg <= 64) {
-            // all pairs (a, b), a < b, flattened over the lanes: row a holds
-            // deg - 1 - a of them, P(a) = a (2 deg - 1 - a) / 2 before it
-            const int total = deg * (deg - 1) / 2;
-            for (int k = lane; k < deg; k += 32) sL[wib][k] = 0;
-            __syncwarp();
-            for (int base = 0; base < total; base += 32) {
-                const int s2 = base + lane;
-                bool cand = false, pass = false;
-                int a = 0, b = 0;
-                if (s2 < total) {
-                    const float D = (float)(2 * deg - 1);
-                    a = (int)((D - sqrtf(D * D - 8.0f * (float)s2)) * 0.5f);
-                    a = max(0, min(a, deg - 2));
-                    while (a > 0 && a * (2 * deg - 1 - a) / 2 > s2) a--;
-                    while (a + 1 <= deg - 2 && (a + 1) * (2 * deg - 2 - a) / 2 <= s2) a++;
-                    b = a + 1 + (s2 - a * (2 * deg - 1 - a) / 2);
-                    const uint32_t v1 = __ldg(&N[a]), v2 = __ldg(&N[b]);
-                    const uint64_t e1 = eoff[v1];
-                    const int deg1 = (int)(eoff[v1 + 1] - e1);
-                    const int pos = lbound(ER + e1, deg1, v2);
-                    cand = pos < deg1 && __ldg(&ER[e1 + pos]) == v2;
-                    if (cand) {
-                        float4 o;
-                        pass = dec_tri<V>(A, pac::ld_ball(&at[v1]), pac::ld_ball(&at[v2]), alpha, o,
-                                          tally);
-                    }
-                    if (pass) atomicOr((unsigned long long *)&sL[wib][a], 1ull << b);
+        for (int c = tid; c < deg; c += kThreads) {
+            const uint32_t x = __ldg(&ER[e0 + c]);
+            S.id[c] = x;
+            S.ball[c] = __ldg(&at[x]);
+            const uint64_t e2 = eoff[x];
+            S.e2[c] = e2;
+            S.d2[c] = (uint16_t)(eoff[x + 1] - e2);
+            S.tab[hash_slot(x, 0, Smem::kBits)] = (uint8_t)c;
+        }
+        for (int k = tid; k < deg * kWords; k += kThreads) S.tri[k] = 0;
+        __syncthreads();
+        const int tries = settle_table(S.tab, S.id, deg, Smem::kBits);
+        // ---- the edges among the neighbours: lanes over the list of N[a]
+        for (int a = wib; a < deg; a += kWarps) {
+            const uint32_t *N2 = ER + S.e2[a];
+            const int deg2 = S.d2[a];
+            uint32_t mine[kWords];
+#pragma unroll
+            for (int w = 0; w < kWords; w++) mine[w] = 0;
+            for (int k = lane; k < deg2; k += 32) {
+                const uint32_t x = __ldg(&N2[k]);
+                const int c = table_find(S.tab, S.id, deg, Smem::kDeg, Smem::kBits, tries, x);
+                const bool hit = c < deg && S.id[c] == x;
+#pragma unroll
+                for (int w = 0; w < kWords; w++)
+                    if (hit && (c >> 5) == w) mine[w] |= 1u << (c & 31);
+            }
+            uint32_t cnt = 0;
+#pragma unroll
+            for (int w = 0; w < kWords; w++) {
+                const uint32_t all = __reduce_or_sync(kFull, mine[w]);
+                if (lane == 0) S.edge[a * kWords + w] = all;
+                cnt += __popc(all);
+            }
+            if (lane == 0) S.rowpre[a + 1] = cnt;
+        }
+        if (tid == 0) {
+            S.rowpre[0] = 0;
+            S.edge[deg * kWords] = 0xffffffffu;  // ends every walk
+        }
+        __syncthreads();
+        if (wib == 0) {
+            uint32_t carry = 0;
+            for (int a0 = 0; a0 < deg; a0 += 32) {
+                const int a = a0 + lane;
+                uint32_t incl = a < deg ? S.rowpre[a + 1] : 0;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= o) incl += v;
                 }
-                const unsigned cm = __ballot_sync(kFull, cand), pm = __ballot_sync(kFull, pass);
-                if (lane == 0) {
-                    cand_acc += __popc(cm);
-                    alpha_acc += __popc(pm);
+                if (a < deg) S.rowpre[a + 1] = carry + incl;
+                carry += __shfl_sync(kFull, incl, 31);
+            }
+        }
+        __syncthreads();
+        // ---- markRealTriangles, an equal share of the candidates per thread
+        const int total = (int)S.rowpre[deg];
+        const int steps = (total + kThreads - 1) / kThreads;
+        const int start = tid * steps, left = max(0, min(total - start, steps));
+        if (left > 0) {
+            int lo = 0, hi = deg;  // rowpre[lo] <= start < rowpre[lo + 1]
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if ((int)S.rowpre[mid] <= start) lo = mid;
+                else hi = mid;
+            }
+            int skip = start - (int)S.rowpre[lo];
+            uint32_t k = (uint32_t)lo * kWords, bits = S.edge[k];
+            for (int q; skip >= (q = __popc(bits)); skip -= q) bits = S.edge[++k];
+            for (; skip > 0; skip--) bits &= bits - 1;
+            for (int s = 0; s < left; s++) {
+                while (!bits) bits = S.edge[++k];
+                const int a = (int)(k / kWords), b = (int)(k % kWords) * 32 + __ffs((int)bits) - 1;
+                bits &= bits - 1;
+                const float4 b1 = S.ball[a], b2 = S.ball[b];
+                float4 o;
+                if (dec_tri<V>(A, Ball{b1.x, b1.y, b1.z, b1.w}, Ball{b2.x, b2.y, b2.z, b2.w}, alpha, o,
+                               tally)) {
+                    atomicOr(&S.tri[k], 1u << (b & 31));
+                    alpha_acc++;
                 }
             }
-            __syncwarp();
-            for (int k = lane; k < deg; k += 32) L[k] = sL[wib][k];
-            __syncwarp();
-            continue;
+            cand_acc += left;
         }
-        for (int a = 0; a < deg - 1; a++) {
-            if (lane < kMaxW) srow[wib][lane] = 0;
-            __syncwarp();
-            const uint32_t v1 = __ldg(&N[a]);
-            const Ball A1 = pac::ld_ball(&at[v1]);
-            const uint32_t *N1 = ER + eoff[v1];
-            const int deg1 = (int)(eoff[v1 + 1] - eoff[v1]);
-            for (int base = a + 1; base < deg; base += 32) {
-                int b = base + lane;
-                bool cand = false, pass = false;
-                if (b < deg) {
-                    uint32_t v2 = __ldg(&N[b]);
-                    int pos = lbound(N1, deg1, v2);
-                    cand = pos < deg1 && __ldg(&N1[pos]) == v2;
-                    if (cand) {
-                        float4 o;
-                        pass = dec_tri<V>(A, A1, pac::ld_ball(&at[v2]), alpha, o, tally);
-                    }
-                }
-                unsigned cm = __ballot_sync(kFull, cand), pm = __ballot_sync(kFull, pass);
-                if (lane == 0) {
-                    cand_acc += __popc(cm);
-                    alpha_acc += __popc(pm);
-                    int w = base >> 6, sh = base & 63;
-                    srow[wib][w] |= (uint64_t)pm << sh;
-                    if (sh > 32 && w + 1 < kMaxW) srow[wib][w + 1] |= (uint64_t)pm >> (64 - sh);
-                }
-                __syncwarp();
-            }
-            if (lane < W) L[(uint64_t)a * W + lane] = srow[wib][lane];
-            __syncwarp();
+        __syncthreads();
+        const int W = (deg + 63) >> 6;
+        uint64_t *L = link + loff[p];
+        for (int k = tid; k < deg * W; k += kThreads) {
+            const int a = k / W, w = k % W;
+            const uint32_t *t = &S.tri[a * kWords + 2 * w];
+            L[k] = (uint64_t)t[0] | (uint64_t)t[1] << 32;
         }
-        if (lane < W) L[(uint64_t)(deg - 1) * W + lane] = 0;
     }
+    const unsigned long long cs = warp_sum(cand_acc), as = warp_sum(alpha_acc);
     flush_tally<V>(tally, ctr);
     if (lane == 0) {
-        bump(ctr, C_CAND_T, cand_acc);
-        bump(ctr, C_ALPHA_T, alpha_acc);
+        bump(ctr, C_CAND_T, cs);
+        bump(ctr, C_ALPHA_T, as);
     }
 }
 
@@ -1232,39 +1335,10 @@ __device__ __forceinline__ void queue_close(const TetQueue &Q, QRes &qr) {
     qr.pos = qr.end;
 }
 
-// The balls of [lo, hi) by class (at most 64, 128, 256 upper neighbours; at
-// least 3): list[class * n ..], counted in ctr[C_CLASS + class].
-__global__ void k_classes(uint64_t lo, uint64_t hi, uint64_t n, const uint64_t *eoff,
-                          const uint64_t *loff, uint64_t *attached, uint32_t *list,
-                          unsigned long long *ctr) {
-    const uint64_t p = lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    const int deg = p < hi ? (int)(eoff[p + 1] - eoff[p]) : 0;
-    if (attached && deg > 0 && deg < 3)  // no class: its rows are not written there
-        for (int a = 0; a < deg; a++) attached[loff[p] + a] = 0;
-    const int mine = deg < 3 ? -1 : deg <= 64 ? 0 : deg <= 128 ? 1 : 2;
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        const unsigned m = __ballot_sync(kFull, mine == c);
-        if (!m) continue;
-        unsigned long long b = 0;
-        if (lane == 0) b = atomicAdd(&ctr[C_CLASS + c], (unsigned long long)__popc(m));
-        b = __shfl_sync(kFull, b, 0);
-        if (mine == c) list[c * n + b + __popc(m & ((1u << lane) - 1))] = (uint32_t)p;
-    }
-}
-
 // How the enumeration treats its inputs: weights and window centres of the
 // exact mode or of the reference's arithmetic, every certified decision
 // replayed or not (verify mode).
 enum : int { kEnumFloat = 0, kEnumExact = 1, kEnumVerify = 2 };
-
-// Slot of ball x in a table of 2^bits, for attempt t: the neighbours of a ball
-// are a few runs of consecutive indices, which the low bits usually keep apart.
-constexpr int kHashTries = 8;
-__device__ __forceinline__ uint32_t hash_slot(uint32_t x, int t, int bits) {
-    return t == 0 ? x & ((1u << bits) - 1) : (x * (2654435769u * (2u * t + 1u))) >> (32 - bits);
-}
 
 // Sum over the coordinates of (binary32 square - square); each difference is
 // exact.
@@ -1424,16 +1498,7 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
         for (int c = tid; c < deg; c += kThreads) wide |= S.d2[c] > 128;
         wide = __syncthreads_or(wide);
         // ---- a table without collisions, so that a lookup is one read
-        int tries = 0;
-        while (true) {
-            bool clash = false;
-            for (int c = tid; c < deg; c += kThreads)
-                clash |= S.tab[hash_slot(S.sN[c], tries, kTabBits)] != (uint8_t)c;
-            if (!__syncthreads_or(clash) || ++tries == kHashTries) break;
-            for (int c = tid; c < deg; c += kThreads)
-                S.tab[hash_slot(S.sN[c], tries, kTabBits)] = (uint8_t)c;
-            __syncthreads();
-        }
+        const int tries = settle_table(S.tab, S.sN, deg, kTabBits);
         // ---- where each neighbour's neighbours stand in p's list: lanes
         // over the list of N[a], one lookup each (the last warp also counts
         // the triangles before each row: its bits but the highest, which has
@@ -1462,19 +1527,7 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
             const int deg2 = S.d2[a];
             for (int k = lane; k < deg2; k += 32) {
                 const uint32_t x = __ldg(&N2[k]);
-                int c;
-                if (tries < kHashTries) {
-                    // a slot no neighbour of p wrote holds anything: the
-                    // comparison settles it
-                    c = S.tab[hash_slot(x, tries, kTabBits)] & (Smem::kDeg - 1);
-                } else {
-                    int hi = deg;
-                    for (c = 0; hi - c > 1;) {
-                        const int mid = (c + hi) >> 1;
-                        if (S.sN[mid] <= x) c = mid;
-                        else hi = mid;
-                    }
-                }
+                const int c = table_find(S.tab, S.sN, deg, Smem::kDeg, kTabBits, tries, x);
                 if (S.sN[c] == x) S.map[a][c] = (uint8_t)k;
             }
         }
@@ -2494,8 +2547,8 @@ static int enumerate(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const TetArg
     int rc = enum_smem_optin<M>(ctx);
     if (rc) return rc;
     const uint64_t balls = hi - lo;
-    k_classes<<<(unsigned)((balls + 255) / 256), 256, 0, s>>>(lo, hi, A.n, A.eoff, A.loff, A.attached, list,
-                                                               A.ctr);
+    k_classes<<<(unsigned)((balls + 255) / 256), 256, 0, s>>>(lo, hi, A.n, A.eoff, A.loff, A.attached, 3,
+                                                               list, A.ctr);
     LAUNCH_CHECK(ctx);
     const unsigned light = (unsigned)std::min<uint64_t>(balls, 148u * (unsigned)std::max(1, cfg.enum_blocks));
     const unsigned heavy = (unsigned)std::min<uint64_t>(balls, 148u * (unsigned)std::max(1, cfg.heavy_blocks));
@@ -2714,10 +2767,24 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
     uint64_t *link = ar.alloc_n<uint64_t>(nL), *faces = ar.alloc_n<uint64_t>(nL);
     if (!link || !faces) return PAC_ERR_OOM;
     CK(cudaMemsetAsync(faces, 0, sizeof(uint64_t) * (nL ? nL : 1), s));
-    CK(cudaMemsetAsync(ctr + C_NEXT, 0, sizeof(unsigned long long), s));
-    k_link<V><<<std::min<unsigned>(warp_blocks(n), 148 * 4), 256, 0, s>>>(n, at, eoff, ER, loff,
-                                                                          link, in.alpha, ctr);
+    uint32_t *classes = ar.alloc_n<uint32_t>(3 * n);  // balls by degree (k_link, enumeration)
+    if (!classes) return PAC_ERR_OOM;
+    k_classes<<<blocks_for(n, 256), 256, 0, s>>>(0, n, n, eoff, loff, nullptr, 2, classes, ctr);
     LAUNCH_CHECK(ctx);
+    const unsigned link_grid = (unsigned)std::min<uint64_t>(n, 148 * 10);
+    if (maxdeg > 128) {
+        k_link<V, kMaxW><<<std::min(link_grid, 148u * 4), 128, 0, s>>>(classes + 2 * n, 2, at, eoff, ER, loff,
+                                                                       link, in.alpha, ctr);
+        LAUNCH_CHECK(ctx);
+    }
+    if (maxdeg > 64) {
+        k_link<V, 2><<<link_grid, 128, 0, s>>>(classes + n, 1, at, eoff, ER, loff, link, in.alpha, ctr);
+        LAUNCH_CHECK(ctx);
+    }
+    if (maxdeg > 1) {
+        k_link<V, 1><<<link_grid, 128, 0, s>>>(classes, 0, at, eoff, ER, loff, link, in.alpha, ctr);
+        LAUNCH_CHECK(ctx);
+    }
     tm.mark();  // 3
 
     // ---- tetrahedra
@@ -2786,8 +2853,7 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
         T.pend = ar.alloc_n<uint2>(T.pend_cap);
         unsigned long long *claim = ar.alloc_n<unsigned long long>(1);
         unsigned long long *ctrA = ar.alloc_n<unsigned long long>(C_NCOUNTERS);
-        uint32_t *classes = ar.alloc_n<uint32_t>(3 * n);  // the enumeration's classes of balls
-        if (!Q.ent || !classes || !T.surv || !T.pend || !claim || !ctrA) return PAC_ERR_OOM;
+        if (!Q.ent || !T.surv || !T.pend || !claim || !ctrA) return PAC_ERR_OOM;
         CK(cudaMemsetAsync(ctr + C_SURV, 0, 2 * sizeof(unsigned long long), s));
         CK(cudaMemsetAsync(ctr + C_INSPHERE, 0, sizeof(unsigned long long), s));
         CK(cudaMemsetAsync(faces, 0, sizeof(uint64_t) * (nL ? nL : 1), s));
