@@ -255,7 +255,7 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--batch-molecules", type=int, default=4096)
     ap.add_argument("--queue-entries", type=int, default=0,
-                    help="cap the alpha-tetrahedron queue (32 B entries; default: a quarter "
+                    help="cap the alpha-tetrahedron queue (8 B entries; default: a quarter "
                          "of free device memory, at most 12 GiB), e.g. to keep a profiled "
                          "run's device memory small")
     ap.add_argument("--no-exact", action="store_true",
@@ -486,7 +486,7 @@ def main():
                            "faster run of each (runs_s)"}
 
     # ---- the precision cascade (PAC_PRED_EXACT): every decision exact, an
-    # FP64 filter with a running error bound and 640-bit integers where it
+    # FP64 filters and integers of up to 640 bits where they
     # cannot tell; throughput on the headline workload and on the 25,000-ball
     # lattice-snapped degeneracy case, with the fallback rates
     exact = None
@@ -501,8 +501,8 @@ def main():
                 ms.append(st_["ms_total"])
             return min(ms), st_
 
-        exact = {"what": "PAC_PRED_EXACT: FP64 filter with a running error bound, 640-bit "
-                         "integer fallback; fallback_rate = exact_fallbacks / filter_evals"}
+        exact = {"what": "PAC_PRED_EXACT: FP64 filters, integer fallback of up to 640 "
+                         "bits; fallback_rate = exact_fallbacks / filter_evals"}
         with pac.Engine(device=local, tet_mode="as-written", predicates="exact") as ex:
             ms, st_ = timed(ex, d_balls.data_ptr(), n, SOL, ALPHA)
             exact["headline_100k"] = {

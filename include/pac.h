@@ -87,8 +87,8 @@ typedef enum {
        working exact fallback): every edge/triangle/tetrahedron alpha test,
        orientation, insphere and attachment test is the exact sign of its
        polynomial in the binary32 inputs, weights (r + sol)^2 taken exactly.
-       Each is decided by a double-precision filter with a running error
-       bound, and by 640-bit integer arithmetic when the filter cannot tell
+       Each is decided by plain double precision with a static bound, else
+       with a running error bound, else by integers of up to 640 bits
        (pac_stats.filter_evals / exact_fallbacks).  Exact zeros of insphere
        go to the simulation of simplicity as in the reference.  Candidate
        sets and windows are the reference's; window centres are computed in
