@@ -26,6 +26,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "certify.cuh"
@@ -1262,14 +1263,17 @@ struct EnumSmem {
     static constexpr int kGroups = 1024;  // triangles listed at a time (one row has fewer)
     static constexpr int kWarps = KW == 1 ? 4 : KW == 2 ? 12 : 16;
     static constexpr int kBlocks = KW == 1 ? 6 : KW == 2 ? 2 : 1;  // per SM
+    // records per warp: a chunk's 32 triangles and one past them, which ends
+    // every walk and which lanes past their share read
+    static constexpr int kRecs = 33;
     float4 rel[kDeg];            // upper neighbours relative to p, and their lifts s
     pac::pencil::Point pt[kDeg]; // the same in double
     uint64_t sL[kDeg * KW];      // p's link rows
     uint64_t e2[kDeg], l2[kDeg]; // per neighbour: its first upper neighbour's index, its link rows
-    GroupRec group[kWarps][33];  // the chunk's triangles, and one past them
+    GroupRec group[kWarps][kRecs];  // the chunk's triangles
     float2 hg[kWarps][kSlots];   // per listed candidate: h, g
-    uint32_t pm[kWarps][33][kWords];  // per triangle: its fourth vertices (bits c); all ones past the last
-    uint32_t face[kWarps][4][32];     // and its row of v2's link matrix (128 bits)
+    uint32_t pm[kWarps][kRecs][kWords];  // per triangle: its fourth vertices (bits c); all ones past the last
+    uint32_t face[kWarps][4][kRecs];     // and its row of v2's link matrix (128 bits)
     uint32_t ring[kWarps][32 * (kRingSteps + 1)];  // queue entries waiting for a full write
     uint16_t cand[kWarps][kSlots];  // listed candidates: group | c << 5 | kCand* bits
     float st[kDeg];              // lifts of the rounded squares
@@ -1283,6 +1287,16 @@ struct EnumSmem {
     uint8_t tab[kTab];           // positions of p's neighbours by a hash of their index
     uint8_t map[kDeg][kDeg];     // [a][c]: position of N[c] in the list of N[a] (alpha edges only)
 };
+// the sweeps index all three by the same record
+template <int KW>
+constexpr bool enum_records_match() {
+    using S = EnumSmem<KW>;
+    constexpr size_t n = S::kRecs;
+    return n == 33 && std::extent<decltype(S::group), 1>::value == n &&
+           std::extent<decltype(S::pm), 1>::value == n && std::extent<decltype(S::face), 2>::value == n;
+}
+static_assert(enum_records_match<1>() && enum_records_match<2>() && enum_records_match<kMaxW>(),
+              "a record past the chunk's last in every array");
 // a listed candidate's alpha test is open; |h| >= hmin (and refutation is on)
 constexpr uint32_t kCandOpen = 1u << 13, kCandSure = 1u << 14;
 
