@@ -1,9 +1,9 @@
 // pipeline.cu -- the single device pass: balls in, weighted alpha complex out.
 //
 // Compiled twice: with -DPAC_NS=pac_strict -fmad=false (IEEE op-by-op, the
-// oracle-identical flavour) and with -DPAC_NS=pac_fma -fmad=true (nvcc's
+// oracle-identical flavour) and with -DPAC_NS=pac_fma -DPAC_CONTRACTED (nvcc's
 // default contraction, the flavour that follows the reference binary built
-// with default flags).  Nothing else differs between the two.
+// with default flags; its fused operations are written out in refarith.cuh).
 //
 // Layout in HBM (n balls, molecules back to back):
 //   at[n]        float4 (x, y, z, r + sol) in (molecule, cell, input index)
@@ -189,7 +189,7 @@ using pac::ex::Tally;
 template <int V>
 __device__ __forceinline__ float wt(float r) {
     if constexpr (V == pac::kExact) return r;
-    else return r * r;
+    else return pac::mul_rn(r, r);
 }
 
 template <int V>
@@ -198,15 +198,16 @@ __device__ __forceinline__ bool dec_edge(const Ball a, const Ball b, float alpha
     else return pac::edge_alpha<V>(a, b, alpha);
 }
 
-// alpha mark of a triangle; the orthosphere (centre, power) goes to o
-template <int V>
+// alpha mark of a triangle; the orthosphere (centre, power) goes to o.  (F, here
+// and below: the place in refarith.cuh whose contraction applies.)
+template <int V, class F>
 __device__ __forceinline__ bool dec_tri(const Ball a, const Ball b, const Ball c, float alpha,
                                         float4 &o, Tally &t) {
     if constexpr (V == pac::kExact) {
         o = make_float4(0.f, 0.f, 0.f, 0.f);
         return pac::ex::tri_alpha(a, b, c, alpha, t);
     } else {
-        return pac::tri_alpha<V>(a, b, c, alpha, o);
+        return pac::tri_alpha<V, F>(a, b, c, alpha, o);
     }
 }
 
@@ -224,10 +225,11 @@ __device__ __forceinline__ float4 tri_sphere(const Ball a, const Ball b, const B
 }
 
 // alpha mark of a tetrahedron; its orthosphere centre goes to o (zeros when
-// the tetrahedron is flat, as in the reference)
-template <int V>
+// the tetrahedron is flat, as in the reference).  wide: a has more than 64
+// upper neighbours.
+template <int V, class F>
 __device__ __forceinline__ bool dec_tet(const Ball a, const Ball b, const Ball c, const Ball d,
-                                        float alpha, float4 &o, Tally &t) {
+                                        float alpha, float4 &o, bool wide, Tally &t) {
     if constexpr (V == pac::kExact) {
         bool flat = false;
         const bool m = pac::ex::tet_alpha(a, b, c, d, alpha, flat, t);
@@ -238,7 +240,7 @@ __device__ __forceinline__ bool dec_tet(const Ball a, const Ball b, const Ball c
         }
         return m;
     } else {
-        return pac::tet_alpha(a, b, c, d, alpha, o);
+        return pac::tet_alpha<F>(a, b, c, d, alpha, o, wide);
     }
 }
 
@@ -253,7 +255,7 @@ __device__ __forceinline__ float dec_orient(const float *pa, const float *pb, co
         return pac::orient3d(pa, pb, pc, pd);
 }
 
-template <int V>
+template <int V, class F>
 __device__ __forceinline__ float dec_insphere(const float *pa, const float *pb, const float *pc,
                                               const float *pd, const float *pe, float wa, float wb,
                                               float wc, float wd, float we, Tally &t) {
@@ -262,7 +264,7 @@ __device__ __forceinline__ float dec_insphere(const float *pa, const float *pb, 
             Ball{pa[0], pa[1], pa[2], wa}, Ball{pb[0], pb[1], pb[2], wb}, Ball{pc[0], pc[1], pc[2], wc},
             Ball{pd[0], pd[1], pd[2], wd}, Ball{pe[0], pe[1], pe[2], we}, t);
     else
-        return pac::insphere_w(pa, pb, pc, pd, pe, wa, wb, wc, wd, we);
+        return pac::insphere_w<F>(pa, pb, pc, pd, pe, wa, wb, wc, wd, we);
 }
 
 // Attachment of the triangle (a0, v1, v2) by ball q; (px, py, pz, cur) is
@@ -777,6 +779,7 @@ __global__ void __launch_bounds__(128) k_link(const uint32_t *list, int cls,
                                               const uint64_t *__restrict__ loff, uint64_t *link,
                                               float alpha, unsigned long long *ctr) {
     using Smem = LinkSmem<KW>;
+    using Place = std::conditional_t<KW == 1, pac::AtLink<V>, pac::AtLinkWide<V>>;
     constexpr int kWords = Smem::kWords, kThreads = 128, kWarps = 4;
     __shared__ Smem S;
     const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
@@ -871,8 +874,8 @@ __global__ void __launch_bounds__(128) k_link(const uint32_t *list, int cls,
                 bits &= bits - 1;
                 const float4 b1 = S.ball[a], b2 = S.ball[b];
                 float4 o;
-                if (dec_tri<V>(A, Ball{b1.x, b1.y, b1.z, b1.w}, Ball{b2.x, b2.y, b2.z, b2.w}, alpha, o,
-                               tally)) {
+                if (dec_tri<V, Place>(A, Ball{b1.x, b1.y, b1.z, b1.w}, Ball{b2.x, b2.y, b2.z, b2.w}, alpha,
+                                      o, tally)) {
                     atomicOr(&S.tri[k], 1u << (b & 31));
                     alpha_acc++;
                 }
@@ -1020,7 +1023,7 @@ __global__ void __launch_bounds__(256) k_tets(TetArgs A) {
                                     const uint32_t v4 = __ldg(&N[c]);
                                     const Ball B4 = pac::ld_ball(&A.at[v4]);
                                     float4 o;
-                                    if (!dec_tet<V>(B1, B2, B3, B4, A.alpha, o, tally)) continue;
+                                    if (!dec_tet<V, pac::AtRun>(B1, B2, B3, B4, A.alpha, o, false, tally)) continue;
                                     if (sweep == 1) alpha_acc++;
                                     if (MODE == 1) {
                                         lane_cnt++;
@@ -1239,6 +1242,9 @@ struct TetQueue {
 };
 constexpr uint32_t kAlphaOpen = 1u << 24;  // the alpha test is left to the scan (counted there)
 constexpr uint32_t kRefuted = 1u << 25;    // refuted: the scan only counts it
+// of pending entries, contracted flavour: see replay_violates; an insphere value
+// was exactly 0
+constexpr uint32_t kDisputed = 1u << 26, kTied = 1u << 27;
 constexpr int kRingSteps = 2;              // candidate steps between writes to the queue
 
 // One triangle of a chunk: pencil::Group and what the sweeps leave.  80 bytes
@@ -1367,13 +1373,13 @@ __device__ __forceinline__ float square_rounding(float x, float y, float z) {
 template <int M>
 __device__ __noinline__ void enum_verify(const TetArgs &A, const MolGrid &G, const float4 b1,
                                          const float4 b2, const float4 b3, const float4 b4,
-                                         int alpha, const float4 *y) {
+                                         bool wide, int alpha, const float4 *y) {
     constexpr int V = (M & kEnumExact) ? pac::kExact : pac::kUpstream;
     Tally tally;
     float4 sph;
     const Ball B1{b1.x, b1.y, b1.z, b1.w}, B2{b2.x, b2.y, b2.z, b2.w}, B3{b3.x, b3.y, b3.z, b3.w},
         B4{b4.x, b4.y, b4.z, b4.w};
-    const bool mark = dec_tet<V>(B1, B2, B3, B4, A.alpha, sph, tally);
+    const bool mark = dec_tet<V, pac::AtEnum>(B1, B2, B3, B4, A.alpha, sph, wide, tally);
     if (alpha >= 0) {
         atomicAdd(&A.ctr[C_CERT], 1ull);
         if (mark != (alpha == 1)) atomicAdd(&A.ctr[C_CERT_BAD], 1ull);
@@ -1384,7 +1390,7 @@ __device__ __noinline__ void enum_verify(const TetArgs &A, const MolGrid &G, con
         const float pe[3] = {y->x, y->y, y->z};
         const float wa = wt<V>(B1.r), wb = wt<V>(B2.r), wc = wt<V>(B3.r), wd = wt<V>(B4.r);
         const float o = dec_orient<V>(pa, pb, pc, pd, wa, wb, wc, wd, tally);
-        const float r = dec_insphere<V>(pa, pb, pc, pd, pe, wa, wb, wc, wd, wt<V>(y->w), tally);
+        const float r = dec_insphere<V, pac::AtScan>(pa, pb, pc, pd, pe, wa, wb, wc, wd, wt<V>(y->w), tally);
         atomicAdd(&A.ctr[C_CERT], 1ull);
         if (!(o < 0 ? r < 0 : r > 0) ||
             !surely_in_window(sph.x, sph.y, sph.z, y->x, y->y, y->z, 0.99f * G.step))
@@ -1707,8 +1713,8 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
                     open_acc += open;
                     if constexpr (M & kEnumVerify)
                         if (face)
-                            enum_verify<M>(A, G, b1, A.at[S.sN[a]], A.at[S.sN[b]], A.at[S.sN[c]], in ? 1 : out ? 0 : -1,
-                                           nullptr);
+                            enum_verify<M>(A, G, b1, A.at[S.sN[a]], A.at[S.sN[b]], A.at[S.sN[c]], KW > 1,
+                                           in ? 1 : out ? 0 : -1, nullptr);
                     const unsigned m = __ballot_sync(kFull, live);
                     if (live) {
                         const int at = n + __popc(m & lt_mask);
@@ -1774,7 +1780,7 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
                                     if (dead)
                                         enum_verify<M>(A, G, b1, A.at[S.sN[R.ab & 0xff]],
                                                        A.at[S.sN[(R.ab >> 8) & 0xff]], A.at[S.sN[c]],
-                                                       -1, &A.at[S.sN[v]]);
+                                                       KW > 1, -1, &A.at[S.sN[v]]);
                             }
                             take = !dead || (e & kCandOpen);
                             if (take)
@@ -1827,6 +1833,85 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
 constexpr int kScanStep = 4;
 constexpr int kScanRefill = 16;  // idle lanes that trigger a refill
 
+// Contracted flavour.  Its lists were first made by an enumeration that
+// refuted a tetrahedron by replaying insphere_w against one suspect: the first of
+// its side of the triangle (a, b) along the pencil among the candidates met so
+// far, or the other side's first.  That replay fused v3's and v4's weights, the
+// scan's rounds them, so a pair within rounding of zero could be a violation there
+// alone, and the lists depend on it.  The scan therefore asks both for what the
+// filter leaves open; a tetrahedron with a ball that violates by the replay only
+// is pending, and k_sos_resolve settles whether that ball was its suspect.
+__device__ __noinline__ bool replay_violates(const float4 *at, uint32_t p, uint32_t v2, uint32_t v3,
+                                             uint32_t v4, uint32_t y) {
+    const float4 a = __ldg(&at[p]), b = __ldg(&at[v2]), c = __ldg(&at[v3]), d = __ldg(&at[v4]),
+                 e = __ldg(&at[y]);
+    const float pa[3] = {a.x, a.y, a.z}, pb[3] = {b.x, b.y, b.z}, pc[3] = {c.x, c.y, c.z},
+                pd[3] = {d.x, d.y, d.z}, pe[3] = {e.x, e.y, e.z};
+    const float o = pac::orient3d(pa, pb, pc, pd), we = pac::mul_rn(e.w, e.w);
+    const float r = pac::insphere_d<pac::AtScan>(
+        pa, pb, pc, pd, pe, pac::sub_rn(pac::mul_rn(a.w, a.w), we), pac::sub_rn(pac::mul_rn(b.w, b.w), we),
+        pac::fma_rn(c.w, c.w, -we), pac::fma_rn(d.w, d.w, -we));
+    return o < 0 ? r < 0 : r > 0;
+}
+
+// Whether that enumeration refuted the tetrahedron of positions a, b, c in p's
+// list.  It took the third vertices of row a 32 at a time and the candidates of
+// those 32 triangles in order, 32 per step; a candidate met the suspects of its
+// own step and of those before.
+__device__ __noinline__ bool replay_refuted(const TetArgs &A, uint32_t p, int a, int b, int c) {
+    const MolGrid &G = A.grids[mol_of(A.mol, p)];
+    if (!A.refute || G.gx > 16384 || G.gy > 16384 || G.gz > 16384) return false;
+    const uint64_t e0 = A.eoff[p];
+    const int deg = (int)(A.eoff[p + 1] - e0), W = (deg + 63) >> 6;
+    const uint32_t *N = A.ER + e0;
+    const uint64_t *L = A.link + A.loff[p];
+    const bool wide = deg > 64;
+    // candidates of the triangle (a, x) in word w
+    auto fourth = [&](int x, int w) {
+        return L[(uint64_t)a * W + w] & L[(uint64_t)x * W + w] & above_mask(x, w);
+    };
+    int third = 0, before = 0, rank = 0;  // b's place in row a; candidates before the triangle; c's place
+    for (int x = a + 1; x < b; x++) third += (int)((L[(uint64_t)a * W + (x >> 6)] >> (x & 63)) & 1ull);
+    for (int x = a + 1, k = 0; x < b; x++) {
+        if (!((L[(uint64_t)a * W + (x >> 6)] >> (x & 63)) & 1ull)) continue;
+        if (k++ >= (third & ~31))
+            for (int w = 0; w < W; w++) before += __popcll(fourth(x, w));
+    }
+    for (int w = 0; w < W; w++) rank += __popcll(fourth(b, w) & ~above_mask(c - 1, w));
+    const int met = ((before + rank) / 32 + 1) * 32 - before;
+    const Ball B1 = pac::ld_ball(&A.at[p]), B2 = pac::ld_ball(&A.at[N[a]]), B3 = pac::ld_ball(&A.at[N[b]]);
+    const float ux = B2.x - B1.x, uy = B2.y - B1.y, uz = B2.z - B1.z;
+    const float vx = B3.x - B1.x, vy = B3.y - B1.y, vz = B3.z - B1.z;
+    const float nx = pac::diff<1>(uy, vz, uz, vy), ny = pac::diff<1>(uz, vx, ux, vz),
+                nz = pac::diff<1>(ux, vy, uy, vx);
+    unsigned long long best[2] = {~0ull, ~0ull};
+    int side_c = -1;
+    float4 sph_c = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int w = 0, i = 0; w < W; w++) {
+        for (uint64_t bits = fourth(b, w); bits && i < met; bits &= bits - 1, i++) {
+            const int x = w * 64 + __ffsll((long long)bits) - 1;
+            const Ball B4 = pac::ld_ball(&A.at[N[x]]);
+            float4 s;
+            pac::tet_alpha<pac::AtEnum>(B1, B2, B3, B4, A.alpha, s, wide);
+            const bool side = pac::plus<1>(pac::sum<1>(nx, B4.x - B1.x, ny, B4.y - B1.y), nz, B4.z - B1.z) > 0.f;
+            float key = pac::plus<1>(pac::sum<1>(nx, s.x, ny, s.y), nz, s.z);
+            if (!side) key = -key;
+            if (!isfinite(key) || (s.x == 0.f && s.y == 0.f && s.z == 0.f)) continue;
+            const uint32_t k = __float_as_uint(key);
+            best[side] = min(best[side], (unsigned long long)((k & 0x80000000u) ? ~k : k | 0x80000000u) << 32 |
+                                             (uint32_t)x);
+            if (x == c) side_c = side, sph_c = s;
+        }
+    }
+    if (side_c < 0) return false;
+    int y = (int)(best[side_c] & 0xffffffffull);
+    if (y == c && best[side_c ^ 1] != ~0ull) y = (int)(best[side_c ^ 1] & 0xffffffffull);
+    if (y == c) return false;
+    const float4 by = A.at[N[y]];
+    return surely_in_window(sph_c.x, sph_c.y, sph_c.z, by.x, by.y, by.z, 0.99f * G.step) &&
+           replay_violates(A.at, p, N[a], N[b], N[c], N[y]);
+}
+
 // k_tets_scan: the empty-orthosphere test (checkTetsOrthosphere,
 // AlphaComplexLargeData.cu:606-734) of the queued tetrahedra.  An entry's
 // orthosphere comes from markRealTets here (or its exact counterpart), which
@@ -1860,7 +1945,7 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 3 : 4) k_tets_scan(Tet
     pac::cert::Insphere ct{};
     int gX = 0, gY = 0, gZ = 0, q = 0;
     uint32_t e = 0, end = 0;
-    bool zero = false;
+    bool zero = false, disputed = false;
     const MolGrid *G = A.grids;
     while (true) {
         // claim: idle lanes take the next entries of the warp's range
@@ -1885,7 +1970,9 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 3 : 4) k_tets_scan(Tet
                 const uint2 en = Q.ent[idx];
                 if (en.x != kNoTet) {
                     p = en.x, key = en.y & 0xffffffu;
-                    const uint32_t *N = A.ER + A.eoff[p];
+                    const uint64_t e0 = A.eoff[p];
+                    const bool wide = pac::kFused && A.eoff[p + 1] - e0 > 64;
+                    const uint32_t *N = A.ER + e0;
                     v2 = __ldg(&N[key & 0xff]), v3 = __ldg(&N[(key >> 8) & 0xff]),
                     v4 = __ldg(&N[key >> 16]);
                     const Ball a1 = pac::ld_ball(&A.at[p]), a2 = pac::ld_ball(&A.at[v2]),
@@ -1907,7 +1994,7 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 3 : 4) k_tets_scan(Tet
                         const float3 x = pac::ex::tet_centre(a1, a2, a3, a4);
                         sph = make_float4(x.x, x.y, x.z, 0.f);
                     } else {
-                        mark = pac::tet_alpha_g(pac::tet_group(a1, a2, a3), a2, a3, a4, A.alpha, sph);
+                        mark = pac::tet_alpha(a1, a2, a3, a4, A.alpha, sph, wide);
                     }
                     if (en.y & kAlphaOpen) {
                         live = mark && !(en.y & kRefuted);
@@ -1933,7 +2020,7 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 3 : 4) k_tets_scan(Tet
                         const int4 cl = window_cell(*G, sph.x, sph.y, sph.z);
                         gX = cl.x, gY = cl.y, gZ = cl.z;
                         q = 0;
-                        zero = false;
+                        zero = disputed = false;
                         window_centre(*G, A.cellbeg, cl, e, end, oob);
                         have = true;
                     }
@@ -1978,13 +2065,16 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 3 : 4) k_tets_scan(Tet
                             Ball{ax, ay, az, wa}, Ball{bx, by, bz, wb}, Ball{cx, cy, cz, wc},
                             Ball{dx, dy, dz, wd}, Ball{bb.x, bb.y, bb.z, we}, tally);
                     } else {
-                        res = dec_insphere<V>(pa, pb, pc, pd, pe, wa, wb, wc, wd, we, tally);
+                        res = dec_insphere<V, pac::AtScan>(pa, pb, pc, pd, pe, wa, wb, wc, wd, we, tally);
                     }
                     const int rdec = (orientation < 0 ? (res < 0) : (res > 0)) ? 1 : 0;
                     if (dec >= 0 && dec != rdec && !(V == pac::kExact && res == 0)) bad++;
                     if (dec < 0) {
                         dec = rdec;
                         if (res == 0) zero = true;
+                        if constexpr (pac::kFused)
+                            if (!rdec && A.refute && !disputed)
+                                disputed = replay_violates(A.at, p, v2, v3, v4, x);
                     }
                 }
                 viol = dec == 1;
@@ -1995,8 +2085,9 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 3 : 4) k_tets_scan(Tet
         bool found = false;
         while (q < kWindowParts && !found) found = window_part(*G, A.cellbeg, gX, gY, gZ, q++, e, end);
         if (!found) {
+            const uint32_t open = pac::kFused ? (disputed ? kDisputed : 0u) | (zero ? kTied : 0u) : 0u;
             emit_survivor(A.eoff, A.ER, A.loff, A.faces, A.surv, A.surv_cap, A.pend, A.pend_cap,
-                          A.ctr, A.tcount, p, key, v2, v3, v4, zero);
+                          A.ctr, A.tcount, p, key | open, v2, v3, v4, zero || disputed);
             have = false;
         }
     }
@@ -2043,7 +2134,13 @@ __global__ void __launch_bounds__(128) k_sos_resolve(TetArgs A, uint64_t npend) 
     for (int k = 0; k < 4; k++) B[k] = pac::ld_ball(&A.at[v[k]]);
     Tally tally;
     float4 sphere;
-    const bool mark = dec_tet<V>(B[0], B[1], B[2], B[3], A.alpha, sphere, tally);
+    const bool mark = dec_tet<V, pac::AtSos>(B[0], B[1], B[2], B[3], A.alpha, sphere, false, tally);
+    bool tied = true;
+    if constexpr (pac::kFused) {
+        tied = pk.y & kTied;
+        if ((pk.y & kDisputed) && replay_refuted(A, (uint32_t)p, a, b, c)) return;
+        pk.y &= 0xffffffu;
+    }
     if (pk.y & kAlphaOpen) {  // its alpha test was left open too
         const bool refuted = pk.y & kRefuted;
         if (lane == 0 && mark) {
@@ -2080,7 +2177,7 @@ __global__ void __launch_bounds__(128) k_sos_resolve(TetArgs A, uint64_t npend) 
     int cc = lin3(gridX, gridY, gridZ, G.gx, G.gy);
     bool viol = false;
     uint32_t calls = 0;
-    for (int q = 0; q < 27 && !viol; q++) {
+    for (int q = 0; q < 27 && tied && !viol; q++) {
         uint32_t beg, end;
         if (q == 0) {
             if (cc < 0 || (uint64_t)cc >= G.ncell) continue;
@@ -2109,8 +2206,8 @@ __global__ void __launch_bounds__(128) k_sos_resolve(TetArgs A, uint64_t npend) 
                     pts[4][1] = atom.y;
                     pts[4][2] = atom.z;
                     ws[4] = wt<V>(atom.r);
-                    float result = dec_insphere<V>(pts[0], pts[1], pts[2], pts[3], pts[4], ws[0], ws[1],
-                                                   ws[2], ws[3], ws[4], tally);
+                    float result = dec_insphere<V, pac::AtSos>(pts[0], pts[1], pts[2], pts[3], pts[4], ws[0],
+                                                               ws[1], ws[2], ws[3], ws[4], tally);
                     zero = result == 0;
                     if (zero) {
                         idx[4] = (int)A.orig[e] + 1;
