@@ -255,7 +255,7 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--batch-molecules", type=int, default=4096)
     ap.add_argument("--queue-entries", type=int, default=0,
-                    help="cap the alpha-tetrahedron queue (8 B entries; default: a quarter "
+                    help="cap the alpha-tetrahedron queue (24 B an entry; default: a quarter "
                          "of free device memory, at most 12 GiB), e.g. to keep a profiled "
                          "run's device memory small")
     ap.add_argument("--no-exact", action="store_true",

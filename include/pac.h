@@ -138,7 +138,8 @@ typedef struct {
     int reserved_i[9];
     /* reserved_u[0]: if nonzero, the number of alpha tetrahedra the pass
        queues per chunk (default: a quarter of free device memory, at most
-       12 GiB, 8 B per entry).  Smaller values force more chunks. */
+       12 GiB, at 24 B per entry: 8 in the queue, 8 in each of the two lists
+       that a whole chunk may end in).  Smaller values force more chunks. */
     uint64_t reserved_u[8];
 } pac_options;
 

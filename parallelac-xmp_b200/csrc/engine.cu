@@ -181,6 +181,7 @@ struct EventSet {
 constexpr pac::LaunchShape kShapes[] = {
     {6, 2, 4, 256}, {5, 2, 4, 256}, {4, 2, 4, 256}, {6, 1, 4, 256}, {6, 2, 3, 256}, {6, 2, 6, 256},
     {6, 2, 4, 128}, {6, 2, 4, 512}, {6, 2, 4, 2048}, {12, 4, 4, 256}, {4, 1, 2, 256}, {6, 4, 4, 64}};
+constexpr uint64_t kEntryBytes = 24;  // of the queue and both lists
 constexpr int kNumShapes = (int)(sizeof(kShapes) / sizeof(kShapes[0]));
 static_assert(kNumShapes <= 16, "Tuner holds 16 timings");
 
@@ -192,16 +193,17 @@ int run(pac_ctx *ctx, const float4 *d_balls, uint64_t n, uint32_t n_mol,
     pac::Ctx &c = ctx->c;
     if (!std::isfinite(sol) || !std::isfinite(alpha))
         return pac::set_error(PAC_ERR_INVALID_ARG, "sol_rad and alpha must be finite");
-    // the alpha-tetrahedron queue: a quarter of the free memory at the
-    // context's first pass, at most 12 GiB (8 B per entry); a pass whose
-    // queued tetrahedra exceed it runs in chunks
+    // the alpha-tetrahedron queue and the survivor and pending lists, each of
+    // which may take in all of a chunk: a quarter of the free memory at the
+    // context's first pass, at most 12 GiB (three times 8 B per entry); a pass
+    // whose queued tetrahedra exceed it runs in chunks
     if (!c.queue_bytes) {
         size_t freeb = 0, totalb = 0;
         cudaMemGetInfo(&freeb, &totalb);
-        c.queue_bytes = std::max<uint64_t>(std::min<uint64_t>(freeb / 4, 12ull << 30), 8ull << 16);
+        c.queue_bytes = std::max<uint64_t>(std::min<uint64_t>(freeb / 4, 12ull << 30), kEntryBytes << 16);
     }
-    uint64_t qbytes = c.queue_bytes;
-    if (c.opt.reserved_u[0]) qbytes = c.opt.reserved_u[0] * 8ull;  // test hook: entries
+    uint64_t entries = c.queue_bytes / kEntryBytes;
+    if (c.opt.reserved_u[0]) entries = c.opt.reserved_u[0];  // test hook
     const pac::LaunchShape *shape = &kShapes[0];
     // launch shapes: the caller's overrides, else the autotuner's current
     // candidate or its choice, else the defaults
@@ -216,7 +218,7 @@ int run(pac_ctx *ctx, const float4 *d_balls, uint64_t n, uint32_t n_mol,
     cfg.formula = c.opt.formula;
     cfg.tet_mode = c.opt.tet_mode;
     cfg.verbose = c.opt.verbose;
-    cfg.queue_entries = qbytes / 8;
+    cfg.queue_entries = entries;
     cfg.exact = c.opt.predicates == PAC_PRED_EXACT;
     cfg.refute = c.opt.reserved_i[5] != 1;
     cfg.slab_world = c.opt.reserved_i[7] > 1 ? c.opt.reserved_i[7] : 1;

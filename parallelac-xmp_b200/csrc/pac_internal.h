@@ -59,7 +59,7 @@ struct PipelineConfig {
     int formula;    // pac_formula
     int tet_mode;   // pac_tet_mode
     int verbose;
-    uint64_t queue_entries;  // alpha tetrahedra queued per chunk (8 B each)
+    uint64_t queue_entries;  // alpha tetrahedra queued per chunk (8 B each, and in both lists)
     bool exact;              // decision-exact predicates (strict flavour only)
     int slab_rank, slab_world;  // one slab of a partition by cell order (world > 1)
     bool refute;             // early refutation in the tetrahedron enumeration
@@ -123,9 +123,9 @@ struct Ctx {
     // events that order it after and before work there (side_stream)
     cudaStream_t side = nullptr;
     cudaEvent_t side_ev[2]{};
-    // bytes for the alpha-tetrahedron queue, fixed at the context's first
-    // pass (a quarter of the memory free then, at most 12 GiB), so that later
-    // passes lay out the pool the same way
+    // bytes for the alpha-tetrahedron queue and the lists its entries end in,
+    // fixed at the context's first pass (a quarter of the memory free then, at
+    // most 12 GiB), so that later passes lay out the pool the same way
     uint64_t queue_bytes = 0;
     Tuner tuner;
 };

@@ -3050,10 +3050,13 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
             if (!scanned) {
                 // every queued tetrahedron becomes at most one survivor or
                 // one pending entry: grow either list (keeping its entries)
-                // first
+                // first; a list of scap entries beside a whole queue's lasts
+                // for all later chunks, so that a list grows once to stay
+                // within its third of the queue's bytes
                 auto grow = [&](uint2 *&list, uint64_t &cap, unsigned long long used) -> int {
                     if (used + queued <= cap) return PAC_OK;
-                    const uint64_t nc = std::max<uint64_t>(2 * cap, used + queued);
+                    const uint64_t need = used + queued;
+                    const uint64_t nc = std::max<uint64_t>(need, std::min<uint64_t>(2 * need, scap + qcap));
                     uint2 *nb = ar.alloc_n<uint2>(nc);
                     if (!nb) return PAC_ERR_OOM;
                     if (used)
