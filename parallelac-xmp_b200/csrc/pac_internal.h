@@ -127,6 +127,7 @@ struct Ctx {
     // fixed at the context's first pass (a quarter of the memory free then, at
     // most 12 GiB), so that later passes lay out the pool the same way
     uint64_t queue_bytes = 0;
+    bool enum_optin = false;  // the enumeration kernels' shared memory is allowed
     Tuner tuner;
 };
 

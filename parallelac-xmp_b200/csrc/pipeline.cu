@@ -2634,18 +2634,19 @@ __global__ void k_mol_rows(uint32_t n_mol, const uint64_t *ball_off, uint64_t n,
 
 // ------------------------------------------------------------------ host
 // The enumeration kernels' shared memory exceeds the static 48 KB: allow it
-// (once per device and flavour; the attribute belongs to the kernel).
+// once per context, whose options fix the kernels it launches (the attribute
+// belongs to the kernel; another context setting it again, on whatever thread,
+// changes nothing).
 template <int M>
 static int enum_smem_optin(pac::Ctx &ctx) {
-    static bool done[64] = {};
-    if (ctx.device >= 0 && ctx.device < 64 && done[ctx.device]) return PAC_OK;
+    if (ctx.enum_optin) return PAC_OK;
     CK(cudaFuncSetAttribute(k_tets_enum<1, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)sizeof(EnumSmem<1>)));
     CK(cudaFuncSetAttribute(k_tets_enum<2, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)sizeof(EnumSmem<2>)));
     CK(cudaFuncSetAttribute(k_tets_enum<kMaxW, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)sizeof(EnumSmem<kMaxW>)));
-    if (ctx.device >= 0 && ctx.device < 64) done[ctx.device] = true;
+    ctx.enum_optin = true;
     return PAC_OK;
 }
 
