@@ -1543,6 +1543,12 @@ __global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBloc
             if (lane == 0) S.rowpre[deg] = base;
         }
         for (int a = wib; a < deg - 2; a += kWarps) {
+            // (rows without a pair of triangles have no candidates: with the
+            // plain-xmp formulas, whose alpha triangles are few, most rows)
+            int nb = 0;
+#pragma unroll
+            for (int w = 0; w < KW; w++) nb += __popcll(S.sL[a * KW + w]);
+            if (nb < 2) continue;
             const uint32_t *N2 = A.ER + S.e2[a];
             const int deg2 = S.d2[a];
             for (int k = lane; k < deg2; k += 32) {
@@ -2345,11 +2351,12 @@ __global__ void __launch_bounds__(256, 4) k_tri_attach(uint64_t p_lo, uint64_t n
                     while (row < deg - 1 && qn < kTQCap - 64) {
                         if (!rloaded) {
 #pragma unroll
-                            for (int w = 0; w < kMaxW; w++)
-                            {
-                                const uint64_t at = lp + (uint64_t)row * W + w;
-                                rbits[w] = w < W ? (link[at] & ~faces[at]) : 0;
-                                if (attached && w < W) rbits[w] &= ~attached[at];
+                            for (int w = 0; w < kMaxW; w++) {
+                                const uint64_t k = lp + (uint64_t)row * W + w;
+                                rbits[w] = w < W ? (link[k] & ~faces[k]) : 0;
+                                // (never with the plain-xmp formulas)
+                                if constexpr (V != pac::kPlainXmp)
+                                    if (attached && w < W) rbits[w] &= ~attached[k];
                             }
                             rloaded = true;
                         }
