@@ -54,8 +54,8 @@ enum Counter {
     C_OOB, C_SURV, C_PEND, C_MAXDEG, C_SOS_RANGE, C_NONFINITE, C_NEXT, C_FILTER, C_FALLBACK,
     C_KILLED, C_KTESTS, C_CERT, C_CERT_BAD,
     C_MAXLEN,                 // largest squared alpha-edge length (bits of a binary32)
-    C_CLASS, C_TAKE = C_CLASS + 3,  // balls per enumeration class, and handed out of each
-    C_NCOUNTERS = C_TAKE + 3
+    C_CLASS, C_TAKE = C_CLASS + 4,  // balls per degree class, and handed out of each
+    C_NCOUNTERS = C_TAKE + 4
 };
 
 struct MolGrid {
@@ -685,19 +685,21 @@ __global__ void __launch_bounds__(256) k_link_size(uint64_t n, const uint32_t *e
     if (top > *(volatile unsigned long long *)&ctr[C_MAXDEG]) atomicMax(&ctr[C_MAXDEG], (unsigned long long)top);
 }
 
-// The balls of [lo, hi) by class (at most 64, 128, 256 upper neighbours; at
-// least `least`): list[class * n ..], counted in ctr[C_CLASS + class].
+// The balls of [lo, hi) by class (0, 1, 2: at most 64, 128, 256 upper neighbours;
+// 3: at most `sparse`; of at least `least`): list[class * n ..], counted in
+// ctr[C_CLASS + class].
+constexpr int kSparse = 3;
 __global__ void k_classes(uint64_t lo, uint64_t hi, uint64_t n, const uint64_t *eoff,
-                          const uint64_t *loff, uint64_t *attached, int least, uint32_t *list,
-                          unsigned long long *ctr) {
+                          const uint64_t *loff, uint64_t *attached, int least, int sparse,
+                          uint32_t *list, unsigned long long *ctr) {
     const uint64_t p = lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const int deg = p < hi ? (int)(eoff[p + 1] - eoff[p]) : 0;
     if (attached && deg > 0 && deg < 3)  // no class: its rows are not written there
         for (int a = 0; a < deg; a++) attached[loff[p] + a] = 0;
-    const int mine = deg < least ? -1 : deg <= 64 ? 0 : deg <= 128 ? 1 : 2;
+    const int mine = deg < least ? -1 : deg <= sparse ? kSparse : deg <= 64 ? 0 : deg <= 128 ? 1 : 2;
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
+    for (int c = 0; c < 4; c++) {
         const unsigned m = __ballot_sync(kFull, mine == c);
         if (!m) continue;
         unsigned long long b = 0;
@@ -890,6 +892,72 @@ __global__ void __launch_bounds__(128) k_link(const uint32_t *list, int cls,
             const uint32_t *t = &S.tri[a * kWords + 2 * w];
             L[k] = (uint64_t)t[0] | (uint64_t)t[1] << 32;
         }
+    }
+    const unsigned long long cs = warp_sum(cand_acc), as = warp_sum(alpha_acc);
+    flush_tally<V>(tally, ctr);
+    if (lane == 0) {
+        bump(ctr, C_CAND_T, cs);
+        bump(ctr, C_ALPHA_T, as);
+    }
+}
+
+// The same for balls of few upper neighbours, a warp per ball: its pairs
+// (a, b) flattened over the lanes, row a's deg - 1 - a of them after the
+// P(a) = a (2 deg - 1 - a) / 2 before it, each looked up by a search in N[a]'s
+// list.  A block spends most of such a ball on barriers and on the chain of
+// loads before them: all links of 231,086 balls without a probe (8.6 upper
+// neighbours on average) 0.60 ms by blocks, 0.29 / 0.25 / 0.235 / 0.24 with balls
+// of at most 12 / 16 / 24 / 32 here; with a probe (41) 1.36 -> 1.33 ms at 100,000.
+// Passes of few balls are as long as their slowest ball and keep to blocks
+// (with 24 here: 28 -> 40 us at 211 balls, 110 -> 120 at 5,003, 396 -> 400 at
+// 25,000 with a probe; 173 -> 87 at 60,000 without).
+constexpr int kLinkWarpDeg = 24;
+constexpr uint64_t kLinkWarpBalls = 1 << 15;
+template <int V>
+__global__ void __launch_bounds__(256) k_link_warp(const uint32_t *list, const float4 *__restrict__ at,
+                                                   const uint64_t *__restrict__ eoff,
+                                                   const uint32_t *__restrict__ ER,
+                                                   const uint64_t *__restrict__ loff, uint64_t *link,
+                                                   float alpha, unsigned long long *ctr) {
+    __shared__ uint32_t rows[8][32];
+    static_assert(kLinkWarpDeg <= 32, "a word per row");
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint64_t count = ctr[C_CLASS + kSparse];
+    uint32_t cand_acc = 0, alpha_acc = 0;
+    Tally tally;
+    for (uint64_t u = warp; u < count; u += nwarps) {
+        const uint32_t p = list[u];
+        const uint64_t e0 = eoff[p];
+        const int deg = (int)(eoff[p + 1] - e0);
+        const uint32_t *N = ER + e0;
+        const Ball A = pac::ld_ball(&at[p]);
+        rows[wib][lane] = 0;
+        __syncwarp();
+        const int total = deg * (deg - 1) / 2;
+        for (int s = lane; s < total; s += 32) {
+            const float D = (float)(2 * deg - 1);
+            int a = (int)((D - sqrtf(D * D - 8.0f * (float)s)) * 0.5f);
+            a = max(0, min(a, deg - 2));
+            while (a > 0 && a * (2 * deg - 1 - a) / 2 > s) a--;
+            while (a + 1 <= deg - 2 && (a + 1) * (2 * deg - 2 - a) / 2 <= s) a++;
+            const int b = a + 1 + (s - a * (2 * deg - 1 - a) / 2);
+            const uint32_t v1 = __ldg(&N[a]), v2 = __ldg(&N[b]);
+            const uint64_t e1 = eoff[v1];
+            const int deg1 = (int)(eoff[v1 + 1] - e1);
+            const int pos = lbound(ER + e1, deg1, v2);
+            if (pos == deg1 || __ldg(&ER[e1 + pos]) != v2) continue;
+            cand_acc++;
+            float4 o;
+            if (dec_tri<V, pac::AtLink<V>>(A, pac::ld_ball(&at[v1]), pac::ld_ball(&at[v2]), alpha, o, tally)) {
+                atomicOr(&rows[wib][a], 1u << b);
+                alpha_acc++;
+            }
+        }
+        __syncwarp();
+        if (lane < deg) link[loff[p] + lane] = rows[wib][lane];
+        __syncwarp();
     }
     const unsigned long long cs = warp_sum(cand_acc), as = warp_sum(alpha_acc);
     flush_tally<V>(tally, ctr);
@@ -2666,7 +2734,7 @@ static int enumerate(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const TetArg
     int rc = enum_smem_optin<M>(ctx);
     if (rc) return rc;
     const uint64_t balls = hi - lo;
-    k_classes<<<(unsigned)((balls + 255) / 256), 256, 0, s>>>(lo, hi, A.n, A.eoff, A.loff, A.attached, 3,
+    k_classes<<<(unsigned)((balls + 255) / 256), 256, 0, s>>>(lo, hi, A.n, A.eoff, A.loff, A.attached, 3, 0,
                                                                list, A.ctr);
     LAUNCH_CHECK(ctx);
     const unsigned light = (unsigned)std::min<uint64_t>(balls, 148u * (unsigned)std::max(1, cfg.enum_blocks));
@@ -2886,10 +2954,16 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
     uint64_t *link = ar.alloc_n<uint64_t>(nL), *faces = ar.alloc_n<uint64_t>(nL);
     if (!link || !faces) return PAC_ERR_OOM;
     CK(cudaMemsetAsync(faces, 0, sizeof(uint64_t) * (nL ? nL : 1), s));
-    uint32_t *classes = ar.alloc_n<uint32_t>(3 * n);  // balls by degree (k_link, enumeration)
+    uint32_t *classes = ar.alloc_n<uint32_t>(4 * n);  // balls by degree (k_link, enumeration)
     if (!classes) return PAC_ERR_OOM;
-    k_classes<<<blocks_for(n, 256), 256, 0, s>>>(0, n, n, eoff, loff, nullptr, 2, classes, ctr);
+    const bool sparse = n >= kLinkWarpBalls;
+    k_classes<<<blocks_for(n, 256), 256, 0, s>>>(0, n, n, eoff, loff, nullptr, 2, sparse ? kLinkWarpDeg : 0,
+                                                 classes, ctr);
     LAUNCH_CHECK(ctx);
+    if (sparse) {
+        k_link_warp<V><<<148 * 8, 256, 0, s>>>(classes + kSparse * n, at, eoff, ER, loff, link, in.alpha, ctr);
+        LAUNCH_CHECK(ctx);
+    }
     const unsigned link_grid = (unsigned)std::min<uint64_t>(n, 148 * 10);
     if (maxdeg > 128) {
         k_link<V, kMaxW><<<std::min(link_grid, 148u * 4), 128, 0, s>>>(classes + 2 * n, 2, at, eoff, ER, loff,
