@@ -912,7 +912,7 @@ __global__ void __launch_bounds__(128) k_link(const uint32_t *list, int cls,
 // (with 24 here: 28 -> 40 us at 211 balls, 110 -> 120 at 5,003, 396 -> 400 at
 // 25,000 with a probe; 173 -> 87 at 60,000 without).
 constexpr int kLinkWarpDeg = 24;
-constexpr uint64_t kLinkWarpBalls = 1 << 15;
+constexpr uint64_t kSparseBalls = 1 << 15;  // (links and enumeration)
 template <int V>
 __global__ void __launch_bounds__(256) k_link_warp(const uint32_t *list, const float4 *__restrict__ at,
                                                    const uint64_t *__restrict__ eoff,
@@ -1328,15 +1328,22 @@ struct GroupRec {
 };
 static_assert(sizeof(GroupRec) == 80, "bank layout");
 
-// KW words per link row: balls of at most 64, 128 or 256 upper neighbours.
-template <int KW>
+// KW words per link row, D neighbours: balls of at most 64, 128 or 256 upper
+// neighbours, or of at most 32 in passes of many balls.  Those have one or two
+// chunks of triangles: a block of one warp each, 20 an SM, instead of four that
+// wait at barriers (enumeration and scan of 231,086 balls without a probe, 2.2
+// triangles an edge: 2.49 -> 1.74 ms; with balls of at most 16 or 24 here 1.80, 1.77;
+// with a probe at 100,000 balls, 41 upper neighbours, 9.01 -> 8.99).  Below
+// kSparseBalls the longest ball counts, and four warps share it (25,000 balls with a
+// probe 2.11 ms, with one warp each 2.18; 211 balls 167 and 231 us).
+template <int KW, int D = 64 * KW>
 struct EnumSmem {
-    static constexpr int kDeg = 64 * KW, kTab = KW == 1 ? 1024 : KW == 2 ? 2048 : 8192;
-    static constexpr int kSlots = KW == 1 ? 216 : 256;  // candidates at a time (one group has fewer)
+    static constexpr int kDeg = D, kTabBits = D == 32 ? 8 : KW == 1 ? 10 : KW == 2 ? 11 : 13;
+    static constexpr int kSlots = D == 32 ? 96 : KW == 1 ? 216 : 256;  // candidates at a time (one group has fewer)
     static constexpr int kWords = 2 * KW;
-    static constexpr int kGroups = 1024;  // triangles listed at a time (one row has fewer)
-    static constexpr int kWarps = KW == 1 ? 4 : KW == 2 ? 12 : 16;
-    static constexpr int kBlocks = KW == 1 ? 6 : KW == 2 ? 2 : 1;  // per SM
+    static constexpr int kGroups = D == 32 ? 512 : 1024;  // triangles listed at a time (one row has fewer)
+    static constexpr int kWarps = D == 32 ? 1 : KW == 1 ? 4 : KW == 2 ? 12 : 16;
+    static constexpr int kBlocks = D == 32 ? 20 : KW == 1 ? 6 : KW == 2 ? 2 : 1;  // per SM
     // records per warp: a chunk's 32 triangles and one past them, which ends
     // every walk and which lanes past their share read
     static constexpr int kRecs = 33;
@@ -1358,18 +1365,19 @@ struct EnumSmem {
     uint16_t tri[kGroups];       // p's triangles: a | b << 8
     pac::pencil::Bounds bounds;  // of the block's ball
     uint16_t d2[kDeg];           // per neighbour: its upper degree
-    uint8_t tab[kTab];           // positions of p's neighbours by a hash of their index
+    uint8_t tab[1 << kTabBits];  // positions of p's neighbours by a hash of their index
     uint8_t map[kDeg][kDeg];     // [a][c]: position of N[c] in the list of N[a] (alpha edges only)
 };
 // the sweeps index all three by the same record
-template <int KW>
+template <int KW, int D = 64 * KW>
 constexpr bool enum_records_match() {
-    using S = EnumSmem<KW>;
+    using S = EnumSmem<KW, D>;
     constexpr size_t n = S::kRecs;
     return n == 33 && std::extent<decltype(S::group), 1>::value == n &&
            std::extent<decltype(S::pm), 1>::value == n && std::extent<decltype(S::face), 2>::value == n;
 }
-static_assert(enum_records_match<1>() && enum_records_match<2>() && enum_records_match<kMaxW>(),
+static_assert(enum_records_match<1, 32>() && enum_records_match<1>() && enum_records_match<2>() &&
+                  enum_records_match<kMaxW>(),
               "a record past the chunk's last in every array");
 // a listed candidate's alpha test is open; |h| >= hmin (and refutation is on)
 constexpr uint32_t kCandOpen = 1u << 13, kCandSure = 1u << 14;
@@ -1500,13 +1508,12 @@ __device__ __noinline__ bool within_reach(const float4 gA, const float4 gC, cons
 
 // A block per ball of one class (list, counted in ctr[C_CLASS + cls], taken
 // from ctr[C_TAKE + cls]).
-template <int KW, int M>
-__global__ void __launch_bounds__(EnumSmem<KW>::kWarps * 32, EnumSmem<KW>::kBlocks)
+template <int KW, int M, int D = 64 * KW>
+__global__ void __launch_bounds__(EnumSmem<KW, D>::kWarps * 32, EnumSmem<KW, D>::kBlocks)
     k_tets_enum(TetArgs A, TetQueue Q, const uint32_t *list, int cls) {
-    using Smem = EnumSmem<KW>;
+    using Smem = EnumSmem<KW, D>;
     constexpr int kWarps = Smem::kWarps, kThreads = kWarps * 32, kSlots = Smem::kSlots;
-    constexpr int kTabBits = KW == 1 ? 10 : KW == 2 ? 11 : 13;
-    static_assert(1 << kTabBits == Smem::kTab, "table size");
+    constexpr int kTabBits = Smem::kTabBits;
 #ifdef PAC_CONTRACTED
     constexpr bool kContracted = !(M & kEnumExact);
 #else
@@ -2734,8 +2741,9 @@ static int enumerate(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const TetArg
     int rc = enum_smem_optin<M>(ctx);
     if (rc) return rc;
     const uint64_t balls = hi - lo;
-    k_classes<<<(unsigned)((balls + 255) / 256), 256, 0, s>>>(lo, hi, A.n, A.eoff, A.loff, A.attached, 3, 0,
-                                                               list, A.ctr);
+    const bool sparse = balls >= kSparseBalls;
+    k_classes<<<(unsigned)((balls + 255) / 256), 256, 0, s>>>(lo, hi, A.n, A.eoff, A.loff, A.attached, 3,
+                                                               sparse ? 32 : 0, list, A.ctr);
     LAUNCH_CHECK(ctx);
     const unsigned light = (unsigned)std::min<uint64_t>(balls, 148u * (unsigned)std::max(1, cfg.enum_blocks));
     const unsigned heavy = (unsigned)std::min<uint64_t>(balls, 148u * (unsigned)std::max(1, cfg.heavy_blocks));
@@ -2758,6 +2766,12 @@ static int enumerate(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const TetArg
     }
     if (maxdeg >= 3) {
         k_tets_enum<1, M><<<light, EnumSmem<1>::kWarps * 32, sizeof(EnumSmem<1>), s>>>(A, Q, list, 0);
+        LAUNCH_CHECK(ctx);
+    }
+    if (sparse) {
+        using Smem = EnumSmem<1, 32>;
+        k_tets_enum<1, M, 32><<<(unsigned)std::min<uint64_t>(balls, 148u * Smem::kBlocks), Smem::kWarps * 32,
+                                sizeof(Smem), s>>>(A, Q, list + kSparse * A.n, kSparse);
         LAUNCH_CHECK(ctx);
     }
     if (aside) CK(cudaStreamWaitEvent(s, ctx.side_ev[1], 0));
@@ -2956,7 +2970,7 @@ static int run_pass_v(pac::Ctx &ctx, const pac::PipelineConfig &cfg, const pac::
     CK(cudaMemsetAsync(faces, 0, sizeof(uint64_t) * (nL ? nL : 1), s));
     uint32_t *classes = ar.alloc_n<uint32_t>(4 * n);  // balls by degree (k_link, enumeration)
     if (!classes) return PAC_ERR_OOM;
-    const bool sparse = n >= kLinkWarpBalls;
+    const bool sparse = n >= kSparseBalls;
     k_classes<<<blocks_for(n, 256), 256, 0, s>>>(0, n, n, eoff, loff, nullptr, 2, sparse ? kLinkWarpDeg : 0,
                                                  classes, ctr);
     LAUNCH_CHECK(ctx);
