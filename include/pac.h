@@ -79,9 +79,10 @@ typedef enum {
        simulation of simplicity on an insphere result of exactly zero
        (predicates.h:4669-5462). */
     PAC_PRED_REFCOMPAT = 0,
-    /* Same, but every operation that the reference leaves to nvcc's default
-       FMA contraction is compiled with contraction enabled (nvcc -fmad=true),
-       to follow the reference binary built with default flags. */
+    /* Same, but with multiply-adds fused as nvcc's default FMA contraction
+       (nvcc -fmad=true) fuses them, to follow the reference binary built with
+       default flags.  Which ones is written out (csrc/refarith.cuh), so the
+       lists do not depend on how this library is compiled. */
     PAC_PRED_REFCOMPAT_FMA = 1,
     /* Exact decisions (no counterpart in the reference, which has no
        working exact fallback): every edge/triangle/tetrahedron alpha test,
@@ -122,7 +123,8 @@ typedef struct {
        no effect (accepted; an earlier enumeration's work units), [4] queue
        entries a scan warp claims (256).
        reserved_i[5] = 1: no early refutation in the enumeration (every
-       alpha tetrahedron goes to the scan; same lists).
+       alpha tetrahedron goes to the scan; same lists, except that with
+       PAC_PRED_REFCOMPAT_FMA a tie within rounding may fall otherwise).
        reserved_i[6] = 1: verify mode -- the enumeration and the scan also
        replay the reference's arithmetic (exact mode: the exact polynomials)
        for every decision that their certified filters take and count
@@ -185,7 +187,9 @@ typedef struct {
     uint64_t sos_calls;       /* insphere results of exactly 0 -> SoS */
     uint64_t exact_fallbacks; /* exact-mode: filter failures -> exact kernel */
     uint64_t filter_evals;    /* exact-mode: filtered decisions */
-    uint64_t ortho_out_of_grid; /* window centres outside the grid */
+    uint64_t ortho_out_of_grid; /* window centres outside the grid, of the
+                                   simplices whose window was visited (the
+                                   enumeration settles most without) */
     uint64_t max_degree;
     /* stage times (CUDA events).  The host entry points copy each list to
        host memory as soon as it is emitted, on a second stream, while the

@@ -218,7 +218,8 @@ class Engine:
         if queue_entries:
             o.reserved_u[0] = int(queue_entries)  # alpha-tetrahedron queue size (testing)
         o.autotune = int(bool(autotune))
-        # launch-shape overrides (include/pac.h, pac_options.reserved_i)
+        # launch-shape overrides (include/pac.h, pac_options.reserved_i;
+        # unit_rows is accepted and has no effect)
         for k, v in enumerate((enum_blocks, scan_blocks, heavy_blocks, unit_rows, scan_claim)):
             if v:
                 o.reserved_i[k] = int(v)

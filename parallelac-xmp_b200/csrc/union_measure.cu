@@ -47,10 +47,6 @@ __device__ __forceinline__ double dot(V3 a, V3 b) { return a.x * b.x + a.y * b.y
 __device__ __forceinline__ V3 cross(V3 a, V3 b) {
     return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
-__device__ __forceinline__ V3 normalize(V3 a) {
-    double l = sqrt(dot(a, a));
-    return l > 0 ? (1.0 / l) * a : a;
-}
 
 constexpr double kPi = 3.14159265358979323846;
 
@@ -109,11 +105,13 @@ struct Terms {
 // axis u to the third centre, the arc inside that ball ends at the triple
 // points, along +-u x w = +-nh of the triple.  The exterior angle of patch i at
 // a triple point is atan2(eta R_i |u_ij x u_im|, R_i^2 u_ij . u_im - t_ij t_im), the same
-// at both points.  With K a template parameter the six circles, four triple
-// points and the sums stay in registers.  One ordered pair at a time, with
+// at both points.  With K a template parameter every index is static, so what the
+// registers hold stays there (at 128 a thread, 0.2 KB of a triangle and 1.5 KB
+// of a tetrahedron spill: see k_union).  One ordered pair at a time, with
 // arrays indexed at run time (local memory), four sines and cosines, three
 // atan2 and normalised tangents per pair: 1.13 ms at 100,008 balls for volume,
-// area and gradients, now 0.56; bound by FP64 issue and latency then and now.
+// area and gradients, now 0.57; bound by FP64 latency then and now (at 40,000
+// balls the tetrahedra issue on 36 % of the cycles with 15 of 64 warps).
 template <int K>
 __device__ __forceinline__ void simplex_terms(const V3 *c, const double *R, Terms &T) {
 #pragma unroll
