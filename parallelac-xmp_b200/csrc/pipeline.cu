@@ -2096,13 +2096,17 @@ __global__ void __launch_bounds__(256, V == pac::kExact ? 3 : 4) k_tets_scan(Tet
                                     pd[3] = {dx, dy, dz};
                         // (exact mode: where the filter's setup accepts it, the
                         // sign of the binary32 value is the exact one)
+                        const int4 cl = window_cell(*G, sph.x, sph.y, sph.z);
                         orientation = pac::orient3d(pa, pb, pc, pd);
+                        // contracted flavour: other minors where the centre names no
+                        // cell (a flat tetrahedron's zero sphere; see refarith.cuh)
+                        if (pac::kFused && (cl.w < 0 || (uint64_t)cl.w >= G->ncell))
+                            orientation = pac::orient3d<0>(pa, pb, pc, pd);
                         ct = pac::cert::setup(ax, ay, az, a1.r * a1.r, bx, by, bz, a2.r * a2.r, cx, cy,
                                               cz, a3.r * a3.r, dx, dy, dz, a4.r * a4.r, orientation,
                                               sph.x, sph.y, sph.z, G->wmax);
                         if (V == pac::kExact && !ct.ok)
                             orientation = dec_orient<V>(pa, pb, pc, pd, wa, wb, wc, wd, tally);
-                        const int4 cl = window_cell(*G, sph.x, sph.y, sph.z);
                         gX = cl.x, gY = cl.y, gZ = cl.z;
                         q = 0;
                         zero = disputed = false;

@@ -16,7 +16,7 @@
 // meets a sum is written with its rounding (diff, sum, plus, minus below), by a
 // sequence per place (the At... structs).  The sequences are those nvcc 12.9
 // gave the kernels that first had this flavour, found by comparing their
-// results -- the spheres of 650,000 tetrahedra bit for bit, 100 million
+// results -- the spheres of 600,000 tetrahedra bit for bit, some 90 million
 // decisions of lattices and clusters whose last radius sits within a few ulps
 // of the decision's flip -- with every choice of sequence.  A place that was
 // compiled twice with two sequences (balls of at most 64 upper neighbours and
@@ -286,7 +286,10 @@ __device__ __forceinline__ bool tet_alpha(const Ball a1, const Ball a2, const Ba
     return le_as_double(dist, alpha);
 }
 
-// orient3d determinant (PRED:2015-2045); the error bound there is dead.
+// orient3d determinant (PRED:2015-2045); the error bound there is dead.  M: its
+// minors (in the empty-orthosphere test they are rounded apart where the
+// window's centre names no cell).
+template <int M = 1>
 __device__ __forceinline__ float orient3d(const float *pa, const float *pb, const float *pc,
                                           const float *pd) {
     float adx = pa[0] - pd[0];
@@ -298,9 +301,9 @@ __device__ __forceinline__ float orient3d(const float *pa, const float *pb, cons
     float adz = pa[2] - pd[2];
     float bdz = pb[2] - pd[2];
     float cdz = pc[2] - pd[2];
-    float bc = diff<1>(bdx, cdy, cdx, bdy);
-    float ca = diff<1>(cdx, ady, adx, cdy);
-    float ab = diff<1>(adx, bdy, bdx, ady);
+    float bc = diff<M>(bdx, cdy, cdx, bdy);
+    float ca = diff<M>(cdx, ady, adx, cdy);
+    float ab = diff<M>(adx, bdy, bdx, ady);
     return plus<1>(sum<1>(adz, bc, bdz, ca), cdz, ab);
 }
 

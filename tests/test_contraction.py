@@ -52,11 +52,16 @@ def inputs(pac, name):
                             "upstream"),
         "plain-sc": lambda: (lattice("sc", 9, 2.47, 1e-5, (1.52, 1.7), near, 105), 0.7, 0.5, "plain-xmp"),
         "plain-sc-near": lambda: (lattice("sc", 9, 1.9, 1e-5, (1.6,), near, 205), 0.3, 0.5, "plain-xmp"),
+        # flat tetrahedra whose window's centre names no cell
+        "sc-flat-beside": lambda: (lattice("sc", 8, 1.908675471852929, 2.6489814044728684e-07, (1.5, 1.6, 1.7),
+                                           (2.230977843233849, 4.63655287871564, -2.0192386464515844), 22009),
+                                   0.0, 0.5, "upstream"),
     }[name]()
 
 
 AS_WRITTEN = ("globule-25013", "globule-25013-far", "globule-10007-far", "globule-60001", "plain-globule-3001",
-              "sc-near", "sc-flat", "sc-far", "bcc-mixed", "fcc-mixed", "sc-wide", "plain-sc", "plain-sc-near")
+              "sc-near", "sc-flat", "sc-far", "bcc-mixed", "fcc-mixed", "sc-wide", "plain-sc", "plain-sc-near",
+              "sc-flat-beside")
 
 
 def sha(a):
