@@ -140,8 +140,8 @@ struct AtRun {  // the same as run
     static constexpr int det[4] = {1, 1, 1, 2}, dist[3] = {2, 1, 0};
 };
 struct AtSos {  // where exact zeros are resolved
-    static constexpr int b1[5] = {1, 1, 1, 1, 1}, b1w[5] = {1, 1, 1, 1, 1};
-    static constexpr int b2[5] = {0, 0, 0, 0, 1}, b3[5] = {2, 2, 2, 0, 0};
+    static constexpr int b1[5] = {1, 1, 1, 0, 0}, b1w[5] = {1, 1, 1, 0, 0};
+    static constexpr int b2[5] = {0, 0, 0, 0, 0}, b3[5] = {2, 2, 2, 0, 0};
     static constexpr int det[4] = {2, 1, 2, 2}, dist[3] = {1, 1, 1};
     static constexpr int dab = 2;
 };

@@ -56,12 +56,22 @@ def inputs(pac, name):
         "sc-flat-beside": lambda: (lattice("sc", 8, 1.908675471852929, 2.6489814044728684e-07, (1.5, 1.6, 1.7),
                                            (2.230977843233849, 4.63655287871564, -2.0192386464515844), 22009),
                                    0.0, 0.5, "upstream"),
+        # zeros whose sphere's cell lies a few last bits from the next
+        "fcc-zeros": lambda: (lattice("fcc", 5, 3.1095230816641637, 2.037890214557819e-06, (1.6,),
+                                      (-0.055745524162997495, 0.20514445427019334, -0.16597770356890662), 31032),
+                              0.7, 0.5, "upstream"),
+        "sc-zeros": lambda: (lattice("sc", 8, 1.8865885658291435, 1.1941421051077662e-06, (1.5, 1.6, 1.7),
+                                     (0.27711935683454136, -0.4374353934075288, 0.05114556876453136), 33084),
+                             0.3, 0.5, "upstream"),
+        "plain-fcc-zeros": lambda: (lattice("fcc", 5, 2.6177705613999813, 8.223267098573607e-08, (1.6,),
+                                            (-2.7772292734515593, -3.878554559071259, 1.7090199477873946), 23053),
+                                    0.7, 0.5, "plain-xmp"),
     }[name]()
 
 
 AS_WRITTEN = ("globule-25013", "globule-25013-far", "globule-10007-far", "globule-60001", "plain-globule-3001",
               "sc-near", "sc-flat", "sc-far", "bcc-mixed", "fcc-mixed", "sc-wide", "plain-sc", "plain-sc-near",
-              "sc-flat-beside")
+              "sc-flat-beside", "fcc-zeros", "sc-zeros", "plain-fcc-zeros")
 
 
 def sha(a):
