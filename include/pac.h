@@ -292,7 +292,7 @@ int pac_union_measure_device(pac_ctx *ctx, const double *d_xyzr, uint32_t n,
    synchronisation).  No counterpart in the reference.  All arguments are as
    for pac_union_measure_device: device balls, a complex with device lists,
    and device gradient buffers -- both or neither; vol/area are host
-   pointers.  Nothing is allocated: the only scratch is a fixed 2 MiB array
+   pointers.  Nothing is allocated: the only scratch is a fixed 3 MiB array
    inside the library that every GPU loading it holds until exit.
    Limit: sum over the four lists of ceil(count / 128) <= 65,536 (about 8.4
    million simplices); larger complexes return PAC_ERR_CAPACITY.  The first

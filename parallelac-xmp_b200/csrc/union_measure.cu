@@ -70,12 +70,14 @@ __device__ __forceinline__ Circle make_circle(V3 a, double Ri, double Rj) {  // 
     return C;
 }
 
-// the two points common to spheres i, j, m: x +- eta nh (x relative to c_i)
+// the two points common to spheres i, j, m: x +- eta nh (x relative to c_i).
+// A complex decided in single precision holds triples whose spheres just miss
+// each other: eta is then 0, or with miss the negative square R^2 - |x|^2.
 struct Triple {
     V3 x, nh;
     double eta, nl;  // nl = |(c_j - c_i) x (c_m - c_i)|
 };
-__device__ __forceinline__ Triple make_triple(V3 a, V3 b, double Ri, double Rj, double Rm) {
+__device__ __forceinline__ Triple make_triple(V3 a, V3 b, double Ri, double Rj, double Rm, bool miss, bool &missing) {
     // a = c_j - c_i, b = c_m - c_i; x in the plane of the centres with equal power
     V3 n = cross(a, b);
     double nn = dot(n, n);
@@ -85,7 +87,9 @@ __device__ __forceinline__ Triple make_triple(V3 a, V3 b, double Ri, double Rj, 
     T.x = (1.0 / nn) * (a1 * cross(b, n) + a2 * cross(n, a));
     T.nl = sqrt(nn);
     T.nh = (1.0 / T.nl) * n;
-    T.eta = sqrt(fmax(Ri * Ri - dot(T.x, T.x), 0.0));
+    const double e2 = Ri * Ri - dot(T.x, T.x);
+    missing |= e2 < 0;
+    T.eta = miss && e2 < 0 ? e2 : sqrt(fmax(e2, 0.0));
     return T;
 }
 
@@ -105,15 +109,23 @@ struct Terms {
 // axis u to the third centre, the arc inside that ball ends at the triple
 // points, along +-u x w = +-nh of the triple.  The exterior angle of patch i at
 // a triple point is atan2(eta R_i |u_ij x u_im|, R_i^2 u_ij . u_im - t_ij t_im), the same
-// at both points.  With K a template parameter every index is static, so what the
+// at both points.  Where the three spheres just miss each other, both points
+// are x, outside the spheres by eps R^2 = |x|^2 - R^2: the arcs vanish or close
+// at the foot of x on the circle, and the angle between the circles' tangent
+// directions there is atan2(eps R^2 |u_ij x u_im|, R^2 u_ij . u_im - t_ij t_im (1 - eps)).
+// With K a template parameter every index is static, so what the
 // registers hold stays there (at 128 a thread, 0.2 KB of a triangle and 1.5 KB
 // of a tetrahedron spill: see k_union).  One ordered pair at a time, with
 // arrays indexed at run time (local memory), four sines and cosines, three
 // atan2 and normalised tangents per pair: 1.13 ms at 100,008 balls for volume,
-// area and gradients, now 0.57; bound by FP64 latency then and now (at 40,000
+// area and gradients, now 0.58; bound by FP64 latency then and now (at 40,000
 // balls the tetrahedra issue on 36 % of the cycles with 15 of 64 warps).
+//
+// Returns whether three of the spheres miss each other: the terms are then right
+// only with miss.
 template <int K>
-__device__ __forceinline__ void simplex_terms(const V3 *c, const double *R, Terms &T) {
+__device__ __forceinline__ bool simplex_terms(const V3 *c, const double *R, bool miss, Terms &T) {
+    bool missing = false;
 #pragma unroll
     for (int i = 0; i < K; i++) {
         T.A[i] = 0;
@@ -150,7 +162,8 @@ __device__ __forceinline__ void simplex_terms(const V3 *c, const double *R, Term
         for (int e = 0; e < kPairs; e++) C[e] = make_circle(c[PJ[e]] - c[PI[e]], R[PI[e]], R[PJ[e]]);
 #pragma unroll
         for (int f = 0; f < kTriples; f++)
-            P[f] = make_triple(c[TB[f]] - c[TA[f]], c[TC[f]] - c[TA[f]], R[TA[f]], R[TB[f]], R[TC[f]]);
+            P[f] = make_triple(c[TB[f]] - c[TA[f]], c[TC[f]] - c[TA[f]], R[TA[f]], R[TB[f]], R[TC[f]], miss,
+                               missing);
         double gb[K];  // sum of arc angle times cosine, and the exterior angles
 #pragma unroll
         for (int i = 0; i < K; i++) gb[i] = 0;
@@ -173,9 +186,11 @@ __device__ __forceinline__ void simplex_terms(const V3 *c, const double *R, Term
                 const V3 nh = s * P[f].nh;
                 const V3 x = c[TA[f]] + P[f].x - o;
                 w[at] = cross(nh, u);
-                b[at] = atan2(P[f].eta, dot(x, w[at]));
+                const double xw = dot(x, w[at]);
+                b[at] = atan2(miss ? fmax(P[f].eta, 0.0) : P[f].eta, xw);
                 E[at][0] = x - P[f].eta * nh;
                 E[at][1] = x + P[f].eta * nh;
+                if (miss && P[f].eta < 0) E[at][0] = E[at][1] = (xw < 0 ? -C[e].rho : C[e].rho) * w[at];
                 at++;
             }
             double phi = 2 * b[0];
@@ -222,7 +237,10 @@ __device__ __forceinline__ void simplex_terms(const V3 *c, const double *R, Term
                 const int f = K == 3 ? 0 : 6 - i - j - m;
                 const double te = i < j ? C[e].ti : C[e].tj, tg = i < m ? C[g].ti : C[g].tj;
                 const double cu = ((i < j) == (i < m) ? 1.0 : -1.0) * dot(C[e].u, C[g].u);
-                const double x = atan2(P[f].eta * P[f].nl * R[i], (R[i] * R[i] * cu - te * tg) * (C[e].d * C[g].d));
+                const double eta = P[f].eta;
+                double y = eta * R[i], tt = te * tg;
+                if (miss && eta < 0) y = -eta, tt += tt * eta / (R[i] * R[i]);
+                const double x = atan2(y * P[f].nl, (R[i] * R[i] * cu - tt) * (C[e].d * C[g].d));
                 gb[i] += K == 3 ? 2 * x : x;
             }
         V3 x0 = {0, 0, 0};
@@ -237,6 +255,7 @@ __device__ __forceinline__ void simplex_terms(const V3 *c, const double *R, Term
         }
         T.V = vol / 3.0;
     }
+    return missing;
 }
 
 // double-double accumulation (TwoSum), so the totals do not depend on the
@@ -284,7 +303,7 @@ __device__ __forceinline__ bool run_sum(unsigned act, uint32_t id, double (&v)[8
 template <int K>
 __global__ void __launch_bounds__(128, K >= 3 ? 4 : 8) k_union(uint64_t ns, const uint32_t *idx, const double4 *balls,
                                                double4 *partial, double *dV, double *dA,
-                                               int want_grad) {
+                                               int want_grad, unsigned *miss) {
     __shared__ double4 wpart[4];
     uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     double vh = 0, vl = 0, ah = 0, al = 0;
@@ -304,7 +323,11 @@ __global__ void __launch_bounds__(128, K >= 3 ? 4 : 8) k_union(uint64_t ns, cons
 #pragma unroll
         for (int q = 0; q < K; q++) c[q] = c[q] - c0;
         Terms T;
-        simplex_terms<K>(c, R, T);
+        const bool missing = simplex_terms<K>(c, R, false, T);
+        if constexpr (K >= 3) {
+            const unsigned m = __ballot_sync(act, missing);
+            if ((threadIdx.x & 31) == 0) miss[4 * blockIdx.x + (threadIdx.x >> 5)] = m;
+        }
         constexpr double sg = (K & 1) ? 1.0 : -1.0;
         vh = sg * T.V;
 #pragma unroll
@@ -330,6 +353,7 @@ __global__ void __launch_bounds__(128, K >= 3 ? 4 : 8) k_union(uint64_t ns, cons
             }
         }
     }
+    if (K >= 3 && !act && (threadIdx.x & 31) == 0) miss[4 * blockIdx.x + (threadIdx.x >> 5)] = 0;
     for (int o = 16; o; o >>= 1) {
         double h1 = __shfl_xor_sync(0xffffffffu, vh, o), l1 = __shfl_xor_sync(0xffffffffu, vl, o);
         double h2 = __shfl_xor_sync(0xffffffffu, ah, o), l2 = __shfl_xor_sync(0xffffffffu, al, o);
@@ -346,6 +370,60 @@ __global__ void __launch_bounds__(128, K >= 3 ? 4 : 8) k_union(uint64_t ns, cons
         }
         partial[blockIdx.x] = r;
     }
+}
+
+// Corrects the terms of the simplices whose spheres just miss each other, one in a
+// million or fewer: a thread per block of k_union reads its four masks and adds,
+// for each bit, the right terms less those that were added.  In k_union itself
+// these cases cost every simplex registers (100,008 balls: 590 to 650 us instead
+// of 560), here 575.
+template <int K>
+__device__ void correct(const uint32_t *id, const double4 *balls, double4 &sum, double *dV, double *dA,
+                        int want_grad) {
+    V3 c[K];
+    double R[K];
+    const double4 b0 = balls[id[0]];
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+        const double4 b = balls[id[q]];
+        R[q] = b.w;
+        c[q] = {b.x - b0.x, b.y - b0.y, b.z - b0.z};
+    }
+#pragma unroll 1
+    for (int w = 0; w < 2; w++) {
+        Terms T;
+        simplex_terms<K>(c, R, w != 0, T);
+        const double sg = ((K & 1) != 0) == (w != 0) ? 1.0 : -1.0;
+        dd_add(sum.x, sum.y, sg * T.V, 0.0);
+#pragma unroll
+        for (int q = 0; q < K; q++) dd_add(sum.z, sum.w, sg * T.A[q], 0.0);
+        if (!want_grad) continue;
+#pragma unroll
+        for (int q = 0; q < K; q++) {
+            double *gv = dV + 4 * (uint64_t)id[q], *ga = dA + 4 * (uint64_t)id[q];
+            const double inv = 2.0 / R[q];
+            atomicAdd(gv, sg * T.M[q].x), atomicAdd(ga, sg * (inv * T.M[q].x + T.rN[q].x));
+            atomicAdd(gv + 1, sg * T.M[q].y), atomicAdd(ga + 1, sg * (inv * T.M[q].y + T.rN[q].y));
+            atomicAdd(gv + 2, sg * T.M[q].z), atomicAdd(ga + 2, sg * (inv * T.M[q].z + T.rN[q].z));
+            atomicAdd(gv + 3, sg * T.A[q]), atomicAdd(ga + 3, sg * (inv * T.A[q] + T.rl[q]));
+        }
+    }
+}
+
+// miss: of the bt blocks of triangles, then of the bq of tetrahedra, as partial
+__global__ void __launch_bounds__(128) k_union_miss(uint32_t bt, const uint32_t *tris, uint32_t bq, const uint32_t *tets,
+                                                    const double4 *balls, double4 *partial, double *dV, double *dA,
+                                                    int want_grad, const unsigned *miss) {
+    const uint32_t b = blockIdx.x * 128 + threadIdx.x;
+    if (b >= bt + bq) return;
+    for (int w = 0; w < 4; w++)
+        for (unsigned m = miss[4 * (uint64_t)b + w]; m; m &= m - 1) {
+            const uint64_t at = 32 * w + (__ffs((int)m) - 1);
+            if (b < bt)
+                correct<3>(tris + 3 * (128 * (uint64_t)b + at), balls, partial[b], dV, dA, want_grad);
+            else
+                correct<4>(tets + 4 * (128 * (uint64_t)(b - bt) + at), balls, partial[b], dV, dA, want_grad);
+        }
 }
 
 __global__ void __launch_bounds__(1024) k_union_total(const double4 *partial, uint64_t np, double *out) {
@@ -376,15 +454,37 @@ __global__ void __launch_bounds__(1024) k_union_total(const double4 *partial, ui
     }
 }
 
-// the kernel of simplices of k vertices
-inline void launch(int k, unsigned blocks, cudaStream_t s, uint64_t ns, const uint32_t *idx,
-                   const double4 *balls, double4 *partial, double *dV, double *dA, int want_grad) {
-    switch (k) {
-        case 1: k_union<1><<<blocks, 128, 0, s>>>(ns, idx, balls, partial, dV, dA, want_grad); break;
-        case 2: k_union<2><<<blocks, 128, 0, s>>>(ns, idx, balls, partial, dV, dA, want_grad); break;
-        case 3: k_union<3><<<blocks, 128, 0, s>>>(ns, idx, balls, partial, dV, dA, want_grad); break;
-        default: k_union<4><<<blocks, 128, 0, s>>>(ns, idx, balls, partial, dV, dA, want_grad);
+// All kernels of one measure on stream s: counts and lists by vertices less one,
+// partial and miss (four words) per block of 128.  Returns the launches.
+inline int launch(cudaStream_t s, const uint64_t (&counts)[4], const uint32_t *const (&lists)[4],
+                  const double4 *balls, double4 *partial, unsigned *miss, double *dV, double *dA, int want_grad,
+                  double *totals) {
+    uint32_t blocks[4], off = 0;
+    int launches = 1;
+    for (int k = 0; k < 4; k++) {
+        const uint32_t nb = blocks[k] = (uint32_t)((counts[k] + 127) / 128);
+        if (!nb) continue;
+        const uint64_t ns = counts[k];
+        const uint32_t *idx = lists[k];
+        double4 *p = partial + off;
+        unsigned *m = miss + 4 * (uint64_t)off;
+        switch (k) {
+            case 0: k_union<1><<<nb, 128, 0, s>>>(ns, idx, balls, p, dV, dA, want_grad, m); break;
+            case 1: k_union<2><<<nb, 128, 0, s>>>(ns, idx, balls, p, dV, dA, want_grad, m); break;
+            case 2: k_union<3><<<nb, 128, 0, s>>>(ns, idx, balls, p, dV, dA, want_grad, m); break;
+            default: k_union<4><<<nb, 128, 0, s>>>(ns, idx, balls, p, dV, dA, want_grad, m);
+        }
+        off += nb;
+        launches++;
     }
+    if (const uint32_t nb = blocks[2] + blocks[3]) {
+        const uint32_t at = blocks[0] + blocks[1];
+        k_union_miss<<<(nb + 127) / 128, 128, 0, s>>>(blocks[2], lists[2], blocks[3], lists[3], balls, partial + at, dV,
+                                                      dA, want_grad, miss + 4 * (uint64_t)at);
+        launches++;
+    }
+    k_union_total<<<1, 1024, 0, s>>>(partial, off, totals);
+    return launches;
 }
 
 }  // namespace pac_union
@@ -408,7 +508,8 @@ int union_measure_device(Ctx &ctx, const double4 *d_balls, uint32_t n, const uin
     uint64_t nblocks = 0;
     for (int k = 0; k < 4; k++) nblocks += (counts[k] + 127) / 128;
     double4 *partial = ctx.arena.alloc_n<double4>(nblocks);
-    if (!acc || !partial || (grad && (!dV || !dA))) return PAC_ERR_OOM;
+    unsigned *miss = ctx.arena.alloc_n<unsigned>(4 * nblocks);
+    if (!acc || !partial || !miss || (grad && (!dV || !dA))) return PAC_ERR_OOM;
     // two timing events, destroyed on every return path
     struct Events {
         cudaEvent_t e[2] = {nullptr, nullptr};
@@ -427,17 +528,7 @@ int union_measure_device(Ctx &ctx, const double4 *d_balls, uint32_t n, const uin
         cudaMemsetAsync(dV, 0, 4 * sizeof(double) * n, s);
         cudaMemsetAsync(dA, 0, 4 * sizeof(double) * n, s);
     }
-    uint64_t off = 0;
-    for (int k = 1; k <= 4; k++) {
-        if (!counts[k - 1]) continue;
-        unsigned blocks = (unsigned)((counts[k - 1] + 127) / 128);
-        pac_union::launch(k, blocks, s, counts[k - 1], lists[k - 1], d_balls, partial + off, dV, dA,
-                          grad ? 1 : 0);
-        ctx.launches++;
-        off += blocks;
-    }
-    pac_union::k_union_total<<<1, 1024, 0, s>>>(partial, off, acc);
-    ctx.launches++;
+    ctx.launches += pac_union::launch(s, counts, lists, d_balls, partial, miss, dV, dA, grad ? 1 : 0, acc);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         cudaStreamSynchronize(s);  // the launches that did start finish first
@@ -467,9 +558,9 @@ int union_measure_device(Ctx &ctx, const double4 *d_balls, uint32_t n, const uin
 // cudaMalloc's implicit device synchronisation.  This entry point allocates
 // nothing: the caller passes the balls, the complex and the gradient buffers
 // in device memory, and the only scratch -- one partial (volume, area) sum
-// per block of 128 simplices and the two totals -- lives in the file-scope
-// array below, which every GPU that loads this library holds until the
-// process exits (2 MiB).
+// and one mask per block of 128 simplices and the two totals -- lives in the
+// file-scope array below, which every GPU that loads this library holds until
+// the process exits (3 MiB).
 //
 // Limit: the four simplex lists together may need at most kNoAllocBlocks
 // blocks of 128, i.e. sum over vertices, edges, triangles and tetrahedra of
@@ -481,8 +572,9 @@ namespace {
 constexpr uint64_t kNoAllocBlocks = 65536;
 constexpr int kMaxDevices = 64;
 
-// partial sums (one double4 per block), then one slot for the two totals
-static __device__ __align__(256) double4 g_noalloc_scratch[kNoAllocBlocks + 1];
+// partial sums (one double4 per block), one slot for the two totals, then the
+// blocks' masks (16 bytes each)
+static __device__ __align__(256) double4 g_noalloc_scratch[kNoAllocBlocks + 1 + kNoAllocBlocks / 2];
 
 std::mutex g_noalloc_mutex;
 double4 *g_noalloc_ptr[kMaxDevices] = {};
@@ -548,18 +640,11 @@ extern "C" int pac_union_measure_noalloc(pac_ctx *ctx, const double *d_xyzr, uin
         cudaMemsetAsync(d_dvol, 0, 4 * sizeof(double) * n, s);
         cudaMemsetAsync(d_darea, 0, 4 * sizeof(double) * n, s);
     }
-    uint64_t off = 0;
-    for (int k = 1; k <= 4; k++) {
-        if (!counts[k - 1]) continue;
-        unsigned nb = (unsigned)((counts[k - 1] + 127) / 128);
-        pac_union::launch(k, nb, s, counts[k - 1], lists[k - 1],
-                          reinterpret_cast<const double4 *>(d_xyzr), scratch + off, d_dvol, d_darea,
-                          grad ? 1 : 0);
-        off += nb;
-    }
-    // every partial slot used is written above; the totals slot is written here
+    // every partial and mask slot used is written; the totals slot is written here
     double *totals = reinterpret_cast<double *>(scratch + kNoAllocBlocks);
-    pac_union::k_union_total<<<1, 1024, 0, s>>>(scratch, off, totals);
+    unsigned *miss = reinterpret_cast<unsigned *>(scratch + kNoAllocBlocks + 1);
+    pac_union::launch(s, counts, lists, reinterpret_cast<const double4 *>(d_xyzr), scratch, miss, d_dvol, d_darea,
+                      grad ? 1 : 0, totals);
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return pac::set_error(PAC_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
